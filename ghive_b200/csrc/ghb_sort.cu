@@ -361,9 +361,9 @@ struct PassParams {
   int8_t dec_vbits[kMaxSortKeys];
   int8_t dec_vshift[kMaxSortKeys];
   int8_t dec_fshift[kMaxSortKeys];
-  uint32_t digit_base[kBins];  // exclusive global offset of each digit
-  uint64_t* status;            // [ntiles][kBins] epoch-tagged look-back words
-  uint32_t epoch;
+  const uint32_t* hist;        // rows of each digit of this pass
+  uint32_t* status;            // [ntiles][kBins] look-back words, zero at the start of the pass
+  uint32_t* status_next;       // the next pass's, zeroed by this one (nullptr: the last pass)
   unsigned long long* counters;
   int32_t* dev_status;
   int32_t spin_limit;          // look-back polls before GHB_ERR_TIMEOUT
@@ -416,24 +416,106 @@ __device__ __forceinline__ void decode_value(const PassParams& p, uint64_t v, in
   }
 }
 
-// Three CTAs per SM: the registers are held to 80 (a few bytes spill), and
-// three CTAs' shared memory fits an SM.
+// A tile's look-back word of one digit: 0 = not published; kTilePrefix | the
+// inclusive count of the digit up to and with this tile (31 bits); else the
+// tile's own count + 1.  Each pass of a call has its own zeroed words.
+constexpr uint32_t kTilePrefix = 0x80000000u;
+constexpr int kTileWindow = 8;   // earlier tiles read at once
+
+__device__ __forceinline__ void tile_store(uint32_t* p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t tile_load(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Rows of digit d in the tiles before `tile`: kTileWindow words are loaded
+// together, so a walk over many unfinished tiles pays one L2 round trip per
+// window and not per tile.  Gives up after `spin_limit` windows that brought
+// nothing new (GHB_ERR_TIMEOUT; the count so far, no larger than the true one).
+__device__ __forceinline__ uint32_t tile_lookback(const uint32_t* words, int64_t tile, int d, int32_t* dev_status,
+                                                  int spin_limit) {
+  uint32_t excl = 0;
+  int64_t t = tile - 1;
+  int spins = 0;
+  while (t >= 0) {
+    uint32_t v[kTileWindow];
+#pragma unroll
+    for (int i = 0; i < kTileWindow; i++) v[i] = t - i >= 0 ? tile_load(words + (t - i) * kBins + d) : kTilePrefix;
+    int used = 0;
+    bool found = false;
+#pragma unroll
+    for (int i = 0; i < kTileWindow; i++) {
+      if (found || used < i || v[i] == 0) continue;   // past the first word not ready
+      used = i + 1;
+      if (v[i] & kTilePrefix) {
+        excl += v[i] & ~kTilePrefix;
+        found = true;
+      } else {
+        excl += v[i] - 1;
+      }
+    }
+    if (found) break;
+    t -= used;
+    if (used == 0 && ++spins >= spin_limit) {
+      raise_status(dev_status, kDevTimeout);
+      break;
+    }
+  }
+  return excl;
+}
+
+// Bound by the shared-memory and load/store data path (80 % busy, DRAM 36 %):
+// about 40 shared wavefronts per 32 rows, 15 more for the global accesses.
+// One pass over 20M packed 64-bit keys with 32-bit values: 148 us (188 us
+// when the look-back read one tile's word at a time, rows past the end were
+// tested per key, and a key's tile position and destination took two table
+// reads each).  Three CTAs per SM (80 registers); measured on the 60M-row
+// sort at this form: 3.57 ms, four CTAs at 64 registers 3.76 (the look-back
+// walks more unfinished tiles), look-back windows of 2 / 4 / 16 tiles 3.57 /
+// 3.50 / 3.9 ms (a 1M-row sort: 0.280 / 0.273 / - against 0.262 ms), ranking
+// by eight ballots 4.37 and by __match_any_sync 4.40 ms, 12 / 18 / 20 / 24
+// keys per thread 4.26 / 3.75 / 3.95 / 3.86 ms.
 template <typename V, int SRC, int DST>
-__global__ void __launch_bounds__(kSortThreads, 3) sort_pass_kernel(PassParams p) {
-  __shared__ uint32_t s_whist[kSortThreads / 32][kBins];  // per-warp counts, then exclusive over warps
-  __shared__ uint32_t s_bexcl[kBins];                      // block-local exclusive offset per digit
-  __shared__ uint64_t s_gbase[kBins];                      // global destination of each digit's run
-  __shared__ uint32_t s_wsum[kSortThreads / 32];
-  __shared__ uint32_t s_match[kSortThreads / 32][kBins];   // lanes of each digit, per warp
+__global__ void __launch_bounds__(kSortThreads, 3) sort_pass_kernel(const __grid_constant__ PassParams p) {
+  constexpr int kWarps = kSortThreads / 32;
+  // per warp and digit: keys ranked so far << 32 | lanes of the item being
+  // ranked, one word so a lane reads both with one load
+  __shared__ unsigned long long s_cnt[kWarps][kBins];
+  __shared__ uint32_t s_pos[kWarps][kBins];   // the warp's first tile position of each digit
+  __shared__ uint32_t s_gb[kBins];       // global destination of each digit's run - its tile position
+  __shared__ uint32_t s_base[kBins];     // global exclusive offset of each digit
+  __shared__ uint32_t s_wsum[kWarps];
   __shared__ int64_t s_tile;
-  extern __shared__ uint64_t s_dyn[];                      // reordered tile: keys, then values
+  extern __shared__ uint64_t s_dyn[];    // reordered tile: its keys, after them its values
   uint64_t* s_keys = s_dyn;
-  V* s_vals = (V*)(s_dyn + kSortTile);
+  V* s_vals = (V*)s_dyn;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
+  const int d = threadIdx.x;             // kSortThreads == kBins: a digit per thread
   const V* vals_in = (const V*)p.vals_in;
   V* vals_out = (V*)p.vals_out;
+
+  // exclusive sum over the 256 digits of v (all threads, two barriers)
+  auto digit_scan = [&](uint32_t v) -> uint32_t {
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (lane == 31) s_wsum[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) before += w < warp ? s_wsum[w] : 0;
+    __syncthreads();
+    return before + incl - v;
+  };
+  s_base[d] = digit_scan(p.hist[d]);
 
   while (true) {
     if (threadIdx.x == 0) {
@@ -451,15 +533,16 @@ __global__ void __launch_bounds__(kSortThreads, 3) sort_pass_kernel(PassParams p
         bulk_prefetch_l2(vals_in + ahead * kSortTile, kSortTile * (uint32_t)sizeof(V));
       }
     }
-    for (int i = threadIdx.x; i < (kSortThreads / 32) * kBins; i += kSortThreads) {
-      (&s_whist[0][0])[i] = 0;
-      (&s_match[0][0])[i] = 0;
-    }
+    for (int i = threadIdx.x; i < kWarps * kBins; i += kSortThreads) (&s_cnt[0][0])[i] = 0;
     __syncthreads();
     const int64_t tile = s_tile;
     if (tile >= p.ntiles) break;
     const int64_t wbase = tile * kSortTile + (int64_t)warp * (32 * kSortItems);
+    const int tile_n = (int)min((int64_t)kSortTile, p.n - tile * kSortTile);
 
+    // Rows past the end carry the key ~0: they are the last of the last
+    // digit, so ranking and reordering take them along at the tile's end and
+    // only the published count leaves them out.
     uint64_t key[kSortItems];
     V val[kSortItems];
     if (SRC == kSrcPacked) {
@@ -467,11 +550,6 @@ __global__ void __launch_bounds__(kSortThreads, 3) sort_pass_kernel(PassParams p
       for (int k = 0; k < kSortItems; k++) {
         int64_t row = wbase + k * 32 + lane;
         key[k] = row < p.n ? __ldcs((const unsigned long long*)p.keys_in + row) : ~0ull;
-      }
-#pragma unroll
-      for (int k = 0; k < kSortItems; k++) {
-        int64_t row = wbase + k * 32 + lane;
-        val[k] = row < p.n ? vals_in[row] : (V)0;
       }
     } else {
       int64_t src[kSortItems];
@@ -499,97 +577,82 @@ __global__ void __launch_bounds__(kSortThreads, 3) sort_pass_kernel(PassParams p
         else val[k] = row < p.n ? (V)ld_raw(p.pay_src, row) : (V)0;
       }
     }
-    // stable rank of each key among the warp's keys with the same digit
-    uint32_t rank[kSortItems];
+    // stable rank of each key among the warp's keys with the same digit: the
+    // lanes holding digit dk set their bits in the digit's word (one shared
+    // atomic, no per-bit ballots), read the word and the running count back,
+    // and the lowest of them clears the one and advances the other
+    uint32_t rank[kSortItems / 2];   // two 16-bit ranks a word
 #pragma unroll
     for (int k = 0; k < kSortItems; k++) {
-      int64_t row = wbase + k * 32 + lane;
-      bool live = row < p.n;
-      uint32_t d = (uint32_t)(key[k] >> p.shift) & (kBins - 1);
-      // the warp's lanes holding digit d: each lane sets its bit in the
-      // digit's word (one shared atomic, no per-bit ballots), reads the word
-      // back, and the lowest of them clears it for the next item
-      unsigned peers = 0;
-      if (live) atomicOr(&s_match[warp][d], 1u << lane);
+      const uint32_t dk = (uint32_t)(key[k] >> p.shift) & (kBins - 1);
+      volatile unsigned long long* word = &s_cnt[warp][dk];
+      atomicOr((unsigned int*)word, 1u << lane);
       __syncwarp();
-      if (live) peers = s_match[warp][d];
+      const unsigned long long w = *word;
+      const uint32_t peers = (uint32_t)w, before = (uint32_t)(w >> 32);
       __syncwarp();
-      if (live && (peers & lt) == 0) s_match[warp][d] = 0;
-      uint32_t before = live ? s_whist[warp][d] : 0;
+      if ((peers & lt) == 0) *word = (unsigned long long)(before + __popc(peers)) << 32;
       __syncwarp();
-      if (live && (peers & lt) == 0) s_whist[warp][d] = before + __popc(peers);
-      __syncwarp();
-      rank[k] = before + __popc(peers & lt);
+      const uint32_t r = before + __popc(peers & lt);
+      rank[k / 2] = k & 1 ? rank[k / 2] | r << 16 : r;
     }
     __syncthreads();
-    // per digit (one thread each): exclusive over warps, block total
-    const int d = threadIdx.x;  // kSortThreads == kBins
+    // per digit (one thread each): exclusive over warps, tile total; publish
+    uint32_t excl_w[kWarps];
     uint32_t total = 0;
 #pragma unroll
-    for (int w = 0; w < kSortThreads / 32; w++) {
-      uint32_t c = s_whist[w][d];
-      s_whist[w][d] = total;
-      total += c;
+    for (int w = 0; w < kWarps; w++) {
+      excl_w[w] = total;
+      total += (uint32_t)(s_cnt[w][d] >> 32);
     }
-    // publish this tile's count of digit d, then look back for its prefix
-    {
-      uint64_t* st = p.status + tile * kBins;
-      uint64_t excl = 0;
-      if (tile == 0) {
-        lb_store(&st[d], lb_pack(p.epoch, kFlagPrefix, total));
-      } else {
-        lb_store(&st[d], lb_pack(p.epoch, kFlagAgg, total));
-        int64_t t = tile - 1;
-        int spins = 0;
-        while (t >= 0) {
-          uint64_t v = lb_load(&p.status[t * kBins + d]);
-          bool ok = ((v >> kEpochShift) & kEpochMask) == (p.epoch & kEpochMask);
-          if (ok && (v & kFlagPrefix)) { excl += v & kCountMask; break; }
-          if (ok && (v & kFlagAgg)) { excl += v & kCountMask; t--; continue; }
-          if (++spins >= p.spin_limit) { raise_status(p.dev_status, kDevTimeout); break; }
-        }
-        lb_store(&st[d], lb_pack(p.epoch, kFlagPrefix, excl + total));
-      }
-      s_gbase[d] = (uint64_t)p.digit_base[d] + excl;
-    }
-    // block-wide exclusive scan of the per-digit totals
-    {
-      uint32_t incl = total;
-      for (int o = 1; o < 32; o <<= 1) {
-        uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-      }
-      if (lane == 31) s_wsum[warp] = incl;
-      __syncthreads();
-      if (warp == 0) {
-        uint32_t v = lane < kSortThreads / 32 ? s_wsum[lane] : 0;
-        uint32_t x = v;
-        for (int o = 1; o < 32; o <<= 1) {
-          uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
-          if (lane >= o) x += t;
-        }
-        if (lane < kSortThreads / 32) s_wsum[lane] = x - v;
-      }
-      __syncthreads();
-      s_bexcl[d] = s_wsum[warp] + incl - total;
-    }
+    const uint32_t mine = d == kBins - 1 ? total - (uint32_t)(kSortTile - tile_n) : total;
+    uint32_t* words = p.status + tile * kBins + d;
+    if (tile == 0) tile_store(words, kTilePrefix | mine);
+    else tile_store(words, mine + 1);
+    if (p.status_next) p.status_next[tile * kBins + d] = 0;   // the next pass's words
+    const uint32_t bexcl = digit_scan(total);
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) s_pos[w][d] = bexcl + excl_w[w];
     __syncthreads();
-    // scatter into shared memory in digit order (stable)
+    // scatter the keys into shared memory in digit order (stable); rank
+    // becomes the tile position
 #pragma unroll
     for (int k = 0; k < kSortItems; k++) {
-      int64_t row = wbase + k * 32 + lane;
-      if (row >= p.n) continue;
-      uint32_t dk = (uint32_t)(key[k] >> p.shift) & (kBins - 1);
-      uint32_t at = s_bexcl[dk] + s_whist[warp][dk] + rank[k];
+      const uint32_t dk = (uint32_t)(key[k] >> p.shift) & (kBins - 1);
+      const uint32_t at = s_pos[warp][dk] + (rank[k / 2] >> (k & 1 ? 16 : 0) & 0xffffu);
       s_keys[at] = key[k];
-      s_vals[at] = val[k];
+      rank[k / 2] = k & 1 ? (rank[k / 2] & 0xffffu) | at << 16 : (rank[k / 2] & 0xffff0000u) | at;
     }
+    // the values are loaded here, when the keys' registers are free, and
+    // arrive during the look-back
+    if (SRC == kSrcPacked) {
+#pragma unroll
+      for (int k = 0; k < kSortItems; k++) {
+        int64_t row = wbase + k * 32 + lane;
+        val[k] = row < p.n ? __ldcs(vals_in + row) : (V)0;
+      }
+    }
+    // look back for the digit's rows in earlier tiles (after the scatter, so
+    // that more of them have published), then publish the prefix
+    uint32_t excl = 0;
+    if (tile > 0) {
+      excl = tile_lookback(p.status, tile, d, p.dev_status, p.spin_limit);
+      tile_store(words, kTilePrefix | (excl + mine));
+    }
+    s_gb[d] = s_base[d] + excl - bexcl;
     __syncthreads();
-    // write runs: element i of the reordered tile goes to gbase[d] + (i - bexcl[d])
-    const int64_t tile_n = min((int64_t)kSortTile, p.n - tile * kSortTile);
+    // write runs: element i of the reordered tile goes to s_gb[digit] + i,
+    // keys first, then the values through the same shared memory
+    uint32_t pos[kSortItems];
+#pragma unroll
+    for (int k = 0; k < kSortItems; k++) {
+      const int i = k * kSortThreads + threadIdx.x;
+      const uint64_t x = s_keys[i];
+      pos[k] = s_gb[(uint32_t)(x >> p.shift) & (kBins - 1)] + (uint32_t)i;
+      if (DST == kDstPacked && i < tile_n) __stcs((unsigned long long*)p.keys_out + pos[k], (unsigned long long)x);
+    }
     if (DST == kDstDecode) {
-      // one key column at a time, its decoding parameters held in registers,
-      // then the carried values
+      // one key column at a time, its decoding parameters held in registers
       for (int j = 0; j < p.K.nkeys; j++) {
         const KeyField& kf = p.K.k[j];
         const int vb = p.dec_vbits[j], vs = p.dec_vshift[j], fs = p.dec_fshift[j];
@@ -598,46 +661,34 @@ __global__ void __launch_bounds__(kSortThreads, 3) sort_pass_kernel(PassParams p
         const bool desc = kf.desc, nf = kf.nulls_first;
         const int type = kf.col.type;
         const ghb_out_column o = p.out_keys[j];
-        for (int i = threadIdx.x; i < tile_n; i += kSortThreads) {
-          const uint64_t k = s_keys[i];
-          const uint32_t dk = (uint32_t)(k >> p.shift) & (kBins - 1);
-          const int64_t pos = (int64_t)(s_gbase[dk] + (i - s_bexcl[dk]));
-          const bool null = fs >= 0 && (((k >> fs) & 1ull) == 0) == nf;
-          uint64_t u = (vb == 0 ? 0 : (k >> vs) & vmask) + umin;
+#pragma unroll
+        for (int k = 0; k < kSortItems; k++) {
+          const int i = k * kSortThreads + threadIdx.x;
+          if (i >= tile_n) continue;
+          const uint64_t x = s_keys[i];
+          const bool null = fs >= 0 && (((x >> fs) & 1ull) == 0) == nf;
+          uint64_t u = (vb == 0 ? 0 : (x >> vs) & vmask) + umin;
           if (desc) u = ~u;
           const int64_t raw = type == GHB_DOUBLE ? (int64_t)unflip_f64_bits(u) : (int64_t)(u ^ 0x8000000000000000ull);
-          write_raw(o, pos, type, raw, null);
+          write_raw(o, pos[k], type, raw, null);
         }
-      }
-      for (int i = threadIdx.x; i < tile_n; i += kSortThreads) {
-        const uint64_t k = s_keys[i];
-        const uint32_t dk = (uint32_t)(k >> p.shift) & (kBins - 1);
-        const int64_t pos = (int64_t)(s_gbase[dk] + (i - s_bexcl[dk]));
-        decode_value(p, (uint64_t)s_vals[i], pos);
-      }
-    } else
-    for (int i = threadIdx.x; i < tile_n; i += kSortThreads) {
-      uint64_t k = s_keys[i];
-      uint32_t dk = (uint32_t)(k >> p.shift) & (kBins - 1);
-      int64_t pos = (int64_t)(s_gbase[dk] + (i - s_bexcl[dk]));
-      if (DST == kDstGather) {
-        gather_write(p, (int64_t)s_vals[i], pos);
-      } else {
-        __stcs((unsigned long long*)p.keys_out + pos, (unsigned long long)k);
-        vals_out[pos] = s_vals[i];
       }
     }
     __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    __threadfence();
-    unsigned long long done = atomicAdd(&p.counters[1], 1ull);
-    if (done == gridDim.x - 1) {
-      p.counters[0] = 0;
-      p.counters[1] = 0;
-      __threadfence();
+#pragma unroll
+    for (int k = 0; k < kSortItems; k++) s_vals[rank[k / 2] >> (k & 1 ? 16 : 0) & 0xffffu] = val[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSortItems; k++) {
+      const int i = k * kSortThreads + threadIdx.x;
+      if (i >= tile_n) continue;
+      if (DST == kDstPacked) __stcs(vals_out + pos[k], s_vals[i]);
+      else if (DST == kDstDecode) decode_value(p, (uint64_t)s_vals[i], pos[k]);
+      else gather_write(p, (int64_t)s_vals[i], pos[k]);
     }
+    __syncthreads();
   }
+  claim_finish(p.counters);
 }
 
 // Output in input order (keys all equal, or n tiny): gathers row r to r, or
@@ -657,7 +708,7 @@ size_t sort_scratch_bytes(int64_t n) {
   size_t b = 0;
   b += 2 * align256((size_t)n * 8);                        // keys ping-pong
   b += 2 * align256((size_t)n * 8);                        // values ping-pong
-  b += align256((size_t)ntiles * kBins * 8);               // look-back status
+  b += 2 * align256((size_t)ntiles * kBins * 4);           // look-back words of two passes
   b += align256((size_t)kMaxSeg * kMaxPasses * kBins * 4); // histograms
   b += align256(3 * 8 * kMaxSortKeys);                     // min/max
   return b + 4096;
@@ -700,7 +751,7 @@ static int32_t set_smem(ghb_ctx* ctx, size_t dyn) {
 // hold the packed keys and values of a one-segment key.
 template <typename V>
 static int32_t run_passes(ghb_ctx* ctx, PassParams& pp, const std::vector<Segment>& segs,
-                          const std::vector<std::vector<int>>& run, const std::vector<uint32_t>& hist,
+                          const std::vector<std::vector<int>>& run, const uint32_t* d_hist,
                           uint64_t* const kb[2], void* const vbv[2], bool packed, cudaStream_t stream) {
   int32_t st;
   int total = 0;
@@ -714,12 +765,13 @@ static int32_t run_passes(ghb_ctx* ctx, PassParams& pp, const std::vector<Segmen
     GHB_LAUNCH_CHECK(ctx);
     return GHB_OK;
   }
-  uint64_t* status = nullptr;
-  size_t status_bytes = (size_t)pp.ntiles * kBins * 8;
-  if ((st = scratch_alloc(ctx, status_bytes, (void**)&status, stream))) return st;
-  GHB_CUDA_TRY(ctx, cudaMemsetAsync(status, 0, status_bytes, stream));
-  pp.status = status;
-  const size_t dyn = (size_t)kSortTile * (8 + sizeof(V));
+  // look-back words: each pass zeroes the ones of the pass after it
+  uint32_t* words[2] = {nullptr, nullptr};
+  const size_t words_bytes = (size_t)pp.ntiles * kBins * 4;
+  for (int i = 0; i < 2; i++)
+    if ((st = scratch_alloc(ctx, words_bytes, (void**)&words[i], stream))) return st;
+  GHB_CUDA_TRY(ctx, cudaMemsetAsync(words[0], 0, words_bytes, stream));
+  const size_t dyn = (size_t)kSortTile * 8;
   if ((st = set_smem<V>(ctx, dyn))) return st;
   int per_sm = 0;
   GHB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -736,18 +788,13 @@ static int32_t run_passes(ghb_ctx* ctx, PassParams& pp, const std::vector<Segmen
       int src = i == 0 ? (have_perm ? kSrcPerm : packed ? kSrcPacked : kSrcCols) : kSrcPacked;
       int dst = last ? (multi ? kDstGather : kDstDecode) : kDstPacked;
       pp.shift = q * kDigitBits;
-      uint32_t acc = 0;
-      const uint32_t* h = &hist[((size_t)s * kMaxPasses + q) * kBins];
-      for (int b = 0; b < kBins; b++) {
-        pp.digit_base[b] = acc;
-        acc += h[b];
-      }
+      pp.hist = d_hist + ((size_t)s * kMaxPasses + q) * kBins;
       pp.keys_in = kb[cur];
       pp.vals_in = vb[cur];
       pp.keys_out = kb[cur ^ 1];
       pp.vals_out = vb[cur ^ 1];
-      // the status region was cleared at the start of this call: tag pass k with k
-      pp.epoch = (uint32_t)done;
+      pp.status = words[done & 1 ? 0 : 1];
+      pp.status_next = last ? nullptr : words[done & 1];
       launch_pass<V>(src, dst, pgrid, dyn, stream, pp);
       GHB_LAUNCH_CHECK(ctx);
       cur ^= 1;
@@ -939,8 +986,8 @@ int32_t sort_impl(ghb_ctx* ctx, const ghb_column* keys, const int32_t* orders,
   pp.dev_status = ctx->d_status;
   pp.spin_limit = ctx->spin_limit;
   const bool packed = !multi;
-  if (wide) return run_passes<uint64_t>(ctx, pp, segs, run, hist, kb, vb, packed, stream);
-  return run_passes<uint32_t>(ctx, pp, segs, run, hist, kb, vb, packed, stream);
+  if (wide) return run_passes<uint64_t>(ctx, pp, segs, run, d_hist, kb, vb, packed, stream);
+  return run_passes<uint32_t>(ctx, pp, segs, run, d_hist, kb, vb, packed, stream);
 }
 
 // ---------------------------------------------------------------- STRING keys
