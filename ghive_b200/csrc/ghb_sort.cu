@@ -10,26 +10,34 @@
 //
 // Pipeline (one call):
 //   1. analyse   one read of the key columns: per key the min/max of its
-//                order image and whether it holds NULLs;
+//                order image and whether it holds NULLs; and a sample of the
+//                packed keys: how many rows share their leading digits;
 //   2. plan      (host) each key becomes sub-fields [null flag][value - min]
 //                of just the width its range needs, packed least-significant
-//                key first into 64-bit segments;
+//                key first into 64-bit segments; and how many leading digits
+//                the radix passes sort by;
 //   3. histogram one read per segment: 8-bit digit histograms of all of the
-//                segment's passes at once; passes whose digit is constant are
-//                skipped;
+//                segment's passes at once; when every digit is sorted by,
+//                passes whose digit is constant are skipped;
 //   4. passes    onesweep-style: each CTA claims a tile, ranks its keys by
 //                digit within each warp (stable: a lane's peers of an item
 //                from one shared atomicOr per lane), gets each digit's global
 //                offset by decoupled look-back over earlier tiles, reorders
-//                the tile in shared memory and writes one run per digit.
+//                the tile in shared memory and writes one run per digit;
+//   5. finish    a one-segment key whose leading digits already set all but a
+//                few rows apart is sorted by those digits only; the finish
+//                puts the rows of each run of equal leading digits in order
+//                (each row counts the rows of its run before it, in shared
+//                memory) and writes the output columns in order.
 // A one-segment key (the common case, e.g. (int32 d, int64 k) with the ranges
-// of the sort workload) is packed by the first pass straight from the user's
-// columns and unpacked by the last pass straight into the output columns; the
+// of the sort workload) is packed by the histogram kernel from the user's
+// columns and unpacked by the finish, or the last pass, into the output columns; the
 // value carried with it is the single payload column, or the row index.  A
 // key wider than 64 bits is sorted segment by segment (least significant
 // first), each later segment packed from the row order the previous one left,
 // and the output is gathered by the final row order.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "ghb_ctx.hpp"
@@ -99,92 +107,255 @@ __device__ __forceinline__ uint64_t sub_bits(const KeySet& K, const SubField& sf
 struct MinMaxParams {
   KeySet K;
   int64_t n;
-  unsigned long long* out;  // per key: [0] min image, [1] max image, [2] any NULL
+  unsigned long long* out;  // per key: [0] max of ~image (~min), [1] max image, [2] any NULL; zeroed
 };
 
-__global__ void __launch_bounds__(256) sort_minmax_kernel(MinMaxParams p) {
-  constexpr int U = 4;
+// Smallest and largest of four or two values (INT, LONG by value; DOUBLE by its
+// order image), NULL sentinels left out.
+struct RawRange {
+  int64_t mn, mx;
+  bool null;
+};
+
+template <int TYPE, bool SENTINEL>
+__device__ __forceinline__ void range_add(RawRange& r, int64_t raw) {
+  if constexpr (SENTINEL) {
+    bool null;
+    if constexpr (TYPE == GHB_INT) null = raw == (int64_t)INT32_MAX;
+    else if constexpr (TYPE == GHB_LONG) null = raw == INT64_MAX;
+    else {
+      const double d = __longlong_as_double(raw);
+      null = d != d;
+    }
+    r.null |= null;
+    if (null) return;
+  }
+  // a double's order image with the sign bit flipped compares as a signed value
+  const int64_t v = TYPE == GHB_DOUBLE ? (int64_t)(flip_f64_bits((uint64_t)raw) ^ 0x8000000000000000ull) : raw;
+  r.mn = min(r.mn, v);
+  r.mx = max(r.mx, v);
+}
+
+// One column by 16-byte loads, U of them in flight per thread (the column is
+// read once, evict-first); its rows past the last whole vector one at a time.
+template <int TYPE, bool SENTINEL>
+__device__ __forceinline__ void range_column(const ghb_column& c, int64_t n, int64_t tid, int64_t stride, RawRange& r) {
+  constexpr int U = 8;
+  using Vec = typename std::conditional<TYPE == GHB_INT, int4, longlong2>::type;
+  constexpr int W = TYPE == GHB_INT ? 4 : 2;
+  const Vec* v = (const Vec*)c.data;
+  const int64_t nv = n / W;
+  auto take = [&](const Vec& x) {
+    if constexpr (TYPE == GHB_INT) {
+      if constexpr (!SENTINEL) {   // 32-bit minima first
+        const int lo = min(min(x.x, x.y), min(x.z, x.w)), hi = max(max(x.x, x.y), max(x.z, x.w));
+        r.mn = min(r.mn, (int64_t)lo);
+        r.mx = max(r.mx, (int64_t)hi);
+      } else {
+        range_add<TYPE, SENTINEL>(r, x.x);
+        range_add<TYPE, SENTINEL>(r, x.y);
+        range_add<TYPE, SENTINEL>(r, x.z);
+        range_add<TYPE, SENTINEL>(r, x.w);
+      }
+    } else {
+      range_add<TYPE, SENTINEL>(r, x.x);
+      range_add<TYPE, SENTINEL>(r, x.y);
+    }
+  };
+  int64_t b = tid;
+  for (; b + (U - 1) * stride < nv; b += U * stride) {
+    Vec x[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) x[u] = __ldcs(v + b + u * stride);
+#pragma unroll
+    for (int u = 0; u < U; u++) take(x[u]);
+  }
+  for (; b < nv; b += stride) take(__ldcs(v + b));
+  for (int64_t q = nv * W + tid; q < n; q += stride) range_add<TYPE, SENTINEL>(r, ld_raw(c, q));
+}
+
+// Reads the key columns once, one after another.  16-byte loads where the
+// column has no NULL map and an aligned base; the minima are taken on the
+// values themselves (32-bit ones for INT) and mapped to order images at the
+// end: (d int32, k int64) of 60M rows 191 us with an image per value, 107 now.
+__global__ void __launch_bounds__(256) sort_minmax_kernel(const __grid_constant__ MinMaxParams p) {
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int j = 0; j < p.K.nkeys; j++) {
     const KeyField& f = p.K.k[j];
-    unsigned long long mn = ~0ull, mx = 0, anynull = 0;
-    auto fold = [&](int64_t raw, int64_t r) {
-      if (f.col.null_mode != GHB_NULLS_NONE && raw_is_null(f.col, raw, r)) {
-        anynull = 1;
-        return;
-      }
-      uint64_t img = key_image(f.col, raw);
-      if (f.desc) img = ~img;
-      mn = min(mn, (unsigned long long)img);
-      mx = max(mx, (unsigned long long)img);
-    };
-    // 16-byte loads, U of them in flight per thread (a column read once,
-    // evict-first); rows past the last whole vector, and columns with a NULL
-    // map or an unaligned base, one value at a time
-    int64_t done = 0;
-    if (f.col.null_mode != GHB_NULLS_BYTEMAP && ((uintptr_t)f.col.data & 15) == 0) {
-      if (f.col.type == GHB_INT) {
-        const int4* v = (const int4*)f.col.data;
-        const int64_t nv = p.n / 4;
-        for (int64_t b = tid; b < nv; b += U * stride) {
-          int4 x[U];
+    const ghb_column& c = f.col;
+    RawRange r{INT64_MAX, INT64_MIN, false};
+    const bool sentinel = c.null_mode == GHB_NULLS_SENTINEL;
+    if (c.null_mode != GHB_NULLS_BYTEMAP && ((uintptr_t)c.data & 15) == 0) {
+      if (c.type == GHB_INT)
+        sentinel ? range_column<GHB_INT, true>(c, p.n, tid, stride, r) : range_column<GHB_INT, false>(c, p.n, tid, stride, r);
+      else if (c.type == GHB_LONG)
+        sentinel ? range_column<GHB_LONG, true>(c, p.n, tid, stride, r) : range_column<GHB_LONG, false>(c, p.n, tid, stride, r);
+      else
+        sentinel ? range_column<GHB_DOUBLE, true>(c, p.n, tid, stride, r) : range_column<GHB_DOUBLE, false>(c, p.n, tid, stride, r);
+    } else {
+      constexpr int U = 4;
+      for (int64_t b = tid; b < p.n; b += U * stride) {
+        int64_t raw[U];
 #pragma unroll
-          for (int u = 0; u < U; u++) x[u] = b + u * stride < nv ? __ldcs(v + b + u * stride) : make_int4(0, 0, 0, 0);
+        for (int u = 0; u < U; u++) raw[u] = b + u * stride < p.n ? ld_raw(c, b + u * stride) : 0;
 #pragma unroll
-          for (int u = 0; u < U; u++) {
-            if (b + u * stride >= nv) continue;
-            fold(x[u].x, 0);
-            fold(x[u].y, 0);
-            fold(x[u].z, 0);
-            fold(x[u].w, 0);
-          }
+        for (int u = 0; u < U; u++) {
+          const int64_t q = b + u * stride;
+          if (q >= p.n) continue;
+          if (raw_is_null(c, raw[u], q)) r.null = true;
+          else if (c.type == GHB_DOUBLE) range_add<GHB_DOUBLE, false>(r, raw[u]);
+          else range_add<GHB_LONG, false>(r, raw[u]);
         }
-        done = nv * 4;
-      } else {
-        const longlong2* v = (const longlong2*)f.col.data;
-        const int64_t nv = p.n / 2;
-        for (int64_t b = tid; b < nv; b += U * stride) {
-          longlong2 x[U];
-#pragma unroll
-          for (int u = 0; u < U; u++) x[u] = b + u * stride < nv ? __ldcs(v + b + u * stride) : make_longlong2(0, 0);
-#pragma unroll
-          for (int u = 0; u < U; u++) {
-            if (b + u * stride >= nv) continue;
-            fold(x[u].x, 0);
-            fold(x[u].y, 0);
-          }
-        }
-        done = nv * 2;
       }
     }
-    for (int64_t r = done + tid; r < p.n; r += stride) fold(ld_raw(f.col, r), r);
     for (int o = 16; o > 0; o >>= 1) {
-      mn = min(mn, __shfl_down_sync(0xffffffffu, mn, o));
-      mx = max(mx, __shfl_down_sync(0xffffffffu, mx, o));
-      anynull |= __shfl_down_sync(0xffffffffu, anynull, o);
+      r.mn = min(r.mn, (int64_t)__shfl_down_sync(0xffffffffu, (long long)r.mn, o));
+      r.mx = max(r.mx, (int64_t)__shfl_down_sync(0xffffffffu, (long long)r.mx, o));
     }
+    const bool wnull = __any_sync(0xffffffffu, r.null);
     // one set of atomics per CTA: every CTA's warps hitting the same three
     // words would serialise at L2
-    __shared__ unsigned long long s_red[3][8];
+    __shared__ int64_t s_red[2][8];
+    __shared__ int s_null[8];
     const int warp = threadIdx.x >> 5;
     if ((threadIdx.x & 31) == 0) {
-      s_red[0][warp] = mn;
-      s_red[1][warp] = mx;
-      s_red[2][warp] = anynull;
+      s_red[0][warp] = r.mn;
+      s_red[1][warp] = r.mx;
+      s_null[warp] = wnull;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+      int64_t mn = r.mn, mx = r.mx;
+      bool null = wnull;
       for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
         mn = min(mn, s_red[0][w]);
         mx = max(mx, s_red[1][w]);
-        anynull |= s_red[2][w];
+        null |= s_null[w] != 0;
       }
-      atomicMin(&p.out[3 * j], mn);
-      atomicMax(&p.out[3 * j + 1], mx);
-      if (anynull) atomicOr(&p.out[3 * j + 2], 1ull);
+      if (mn <= mx) {
+        // order images (a value's sign bit flipped); DESC complements them
+        uint64_t lo = flip_i64(mn), hi = flip_i64(mx);
+        if (f.desc) {
+          const uint64_t t = ~lo;
+          lo = ~hi;
+          hi = t;
+        }
+        atomicMax(&p.out[3 * j], (unsigned long long)~lo);
+        atomicMax(&p.out[3 * j + 1], (unsigned long long)hi);
+      }
+      if (null) atomicOr(&p.out[3 * j + 2], 1ull);
     }
     __syncthreads();
+  }
+}
+
+// Range of a key's order images from its three words; false: no value.
+__host__ __device__ __forceinline__ bool key_range(const unsigned long long* mm, uint64_t* umin, uint64_t* range) {
+  const uint64_t lo = ~mm[0], hi = mm[1];
+  const bool any = lo <= hi;
+  *umin = any ? lo : 0;
+  *range = any ? hi - lo : 0;
+  return any;
+}
+
+// ---------------------------------------------------------------- sample
+// Ordered pairs of sampled rows whose packed keys share their leading q
+// digits, for q = first..8 (pairs[q]): each CTA packs S random rows' keys (the
+// ranges are on the device already) into shared memory and compares 64 of them
+// with all.  pairs[q] / S^2 is the chance that two rows share a run of equal
+// leading digits.  A key wider than 64 bits is not sampled.
+constexpr int kSampleMax = 2048;
+constexpr int kSampleRows = 64;   // rows a CTA compares with all
+
+struct SampleParams {
+  KeySet K;
+  int64_t n;
+  int32_t S;               // rows sampled: 1024 or 2048
+  int32_t first;           // fewest leading digits worth counting, at most 4
+  const unsigned long long* mm;
+  unsigned long long* pairs;   // [9], zeroed
+};
+
+__global__ void __launch_bounds__(256) sort_sample_kernel(const __grid_constant__ SampleParams p) {
+  __shared__ uint64_t s_key[kSampleMax];
+  __shared__ __align__(16) uint32_t s_hi[kSampleMax];   // the keys' upper halves
+  __shared__ uint64_t s_umin[kMaxSortKeys];
+  __shared__ int s_vshift[kMaxSortKeys], s_fshift[kMaxSortKeys], s_total;
+  __shared__ unsigned int s_pairs[9];
+  if (threadIdx.x < 9) s_pairs[threadIdx.x] = 0;
+  if (threadIdx.x == 0) {
+    int bits = 0;
+    for (int j = p.K.nkeys - 1; j >= 0; j--) {
+      uint64_t range;
+      key_range(p.mm + 3 * j, &s_umin[j], &range);
+      s_vshift[j] = bits;
+      bits += range == 0 ? 0 : 64 - __clzll((long long)range);
+      s_fshift[j] = p.mm[3 * j + 2] ? bits++ : -1;
+    }
+    s_total = bits;
+  }
+  __syncthreads();
+  const int total = s_total;
+  if (total > 64 || total <= 8 * p.first) return;
+  constexpr int U = 4;
+  for (int base = threadIdx.x; base < p.S; base += U * blockDim.x) {   // S is a multiple of U * blockDim.x
+    int64_t row[U];
+    uint64_t k[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      row[u] = (int64_t)__umul64hi(mix64((uint64_t)(base + u * blockDim.x) + 1), (uint64_t)p.n);
+      k[u] = 0;
+    }
+    for (int j = 0; j < p.K.nkeys; j++) {
+      const KeyField& f = p.K.k[j];
+      int64_t raw[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) raw[u] = ld_raw(f.col, row[u]);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const bool null = f.col.null_mode != GHB_NULLS_NONE && raw_is_null(f.col, raw[u], row[u]);
+        uint64_t v = key_image(f.col, raw[u]);
+        if (f.desc) v = ~v;
+        if (!null && s_vshift[j] < 64) k[u] |= (v - s_umin[j]) << s_vshift[j];
+        if (s_fshift[j] >= 0 && null != (bool)f.nulls_first) k[u] |= 1ull << s_fshift[j];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint64_t x = k[u] << (64 - total);
+      s_key[base + u * blockDim.x] = x;
+      s_hi[base + u * blockDim.x] = (uint32_t)(x >> 32);
+    }
+  }
+  __syncthreads();
+  unsigned int cnt[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};   // pairs with exactly q equal leading digits
+  const int me = blockIdx.x * kSampleRows + threadIdx.x % kSampleRows;
+  const uint64_t x = s_key[me];
+  const uint32_t xh = (uint32_t)(x >> 32), lead = 0xffffffffu << (32 - 8 * p.first);
+  const int span = p.S / (256 / kSampleRows), j0 = (threadIdx.x / kSampleRows) * span;
+#pragma unroll 4
+  for (int j = j0; j < j0 + span; j += 4) {
+    const uint4 y = *(const uint4*)&s_hi[j];
+    const bool hit[4] = {((xh ^ y.x) & lead) == 0, ((xh ^ y.y) & lead) == 0, ((xh ^ y.z) & lead) == 0,
+                         ((xh ^ y.w) & lead) == 0};
+    if (!(hit[0] | hit[1] | hit[2] | hit[3])) continue;
+    for (int e = 0; e < 4; e++) {
+      if (((xh ^ s_hi[j + e]) & lead) || j + e == me) continue;
+      const uint64_t diff = x ^ s_key[j + e];
+      const int q = diff == 0 ? 8 : __clzll((long long)diff) / 8;
+#pragma unroll
+      for (int k = 0; k < 9; k++) cnt[k] += k == q;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 9; k++)
+    if (cnt[k]) atomicAdd(&s_pairs[k], cnt[k]);
+  __syncthreads();
+  if (threadIdx.x >= (unsigned)p.first && threadIdx.x < 9) {
+    unsigned long long v = 0;   // at least q equal leading digits
+    for (int k = threadIdx.x; k < 9; k++) v += s_pairs[k];
+    if (v) atomicAdd(&p.pairs[threadIdx.x], v);
   }
 }
 
@@ -220,6 +391,7 @@ struct HistParams {
   SubPlan sub[kMaxSub];     // the segment's sub-fields, self-contained
   int64_t n;
   int32_t npasses;
+  int32_t shift0;  // the first pass's digit starts here (lower bits are left to the finish)
   uint32_t* hist;  // [npasses][kBins]
   // a one-segment key: the packed keys and carried values are written here
   // too, so every radix pass reads packed keys
@@ -276,7 +448,8 @@ __global__ void __launch_bounds__(256) sort_hist_kernel(HistParams p) {
       }
 #pragma unroll
       for (int u = 0; u < 4; u++)
-        for (int q = 0; q < p.npasses; q++) atomicAdd(&sh[q][(k[u] >> (q * kDigitBits)) & (kBins - 1)], 1u);
+        for (int q = 0; q < p.npasses; q++)
+          atomicAdd(&sh[q][(k[u] >> (p.shift0 + q * kDigitBits)) & (kBins - 1)], 1u);
       if (p.keys_out) {
         ulonglong2* ko = (ulonglong2*)(p.keys_out + r);
         __stcs(ko, make_ulonglong2(k[0], k[1]));
@@ -319,7 +492,8 @@ __global__ void __launch_bounds__(256) sort_hist_kernel(HistParams p) {
     for (int u = 0; u < U; u++) {
       const int64_t r = base + u * stride;
       if (r >= p.n) continue;
-      for (int q = 0; q < p.npasses; q++) atomicAdd(&sh[q][(k[u] >> (q * kDigitBits)) & (kBins - 1)], 1u);
+      for (int q = 0; q < p.npasses; q++)
+        atomicAdd(&sh[q][(k[u] >> (p.shift0 + q * kDigitBits)) & (kBins - 1)], 1u);
       if (p.keys_out) {
         __stcs((unsigned long long*)p.keys_out + r, (unsigned long long)k[u]);
         const uint64_t v = p.carry_rowid ? (uint64_t)r : (uint64_t)ld_raw(p.pay_src, r);
@@ -367,6 +541,7 @@ struct PassParams {
   unsigned long long* counters;
   int32_t* dev_status;
   int32_t spin_limit;          // look-back polls before GHB_ERR_TIMEOUT
+  uint32_t* long_runs;         // the finish: [0] runs it leaves to sort_finish_long_kernel, then their first rows
 };
 
 __device__ __forceinline__ void write_raw(const ghb_out_column& o, int64_t pos, int type, int64_t raw,
@@ -691,6 +866,433 @@ __global__ void __launch_bounds__(kSortThreads, 3) sort_pass_kernel(const __grid
   claim_finish(p.counters);
 }
 
+// ---------------------------------------------------------------- finish
+// Writes raw[k] (NULL: bit k of `nulls`) to row pos[k] of an output column, k
+// with bit k of `live`: the type and the NULL map are tested once per column.
+template <int N>
+__device__ __forceinline__ void put_rows(const ghb_out_column& o, int type, const int64_t (&raw)[N], uint32_t nulls,
+                                         const uint32_t (&pos)[N], uint32_t live) {
+  if (type == GHB_INT) {
+#pragma unroll
+    for (int k = 0; k < N; k++)
+      if (live >> k & 1) ((int32_t*)o.data)[pos[k]] = nulls >> k & 1 ? INT32_MAX : (int32_t)raw[k];
+  } else {
+    const int64_t none = type == GHB_LONG ? INT64_MAX : 0x7ff8000000000000ll;
+#pragma unroll
+    for (int k = 0; k < N; k++)
+      if (live >> k & 1) ((int64_t*)o.data)[pos[k]] = nulls >> k & 1 ? none : raw[k];
+  }
+  if (o.is_null) {
+#pragma unroll
+    for (int k = 0; k < N; k++)
+      if (live >> k & 1) o.is_null[pos[k]] = nulls >> k & 1;
+  }
+}
+
+// Bit k: raw[k] of row row[k] is NULL.
+template <int N>
+__device__ __forceinline__ uint32_t null_bits(const ghb_column& c, const int64_t (&raw)[N], const int64_t (&row)[N],
+                                              uint32_t live) {
+  uint32_t m = 0;
+  if (c.null_mode == GHB_NULLS_NONE) return 0;
+#pragma unroll
+  for (int k = 0; k < N; k++)
+    if (live >> k & 1) m |= (raw_is_null(c, raw[k], row[k]) ? 1u : 0u) << k;
+  return m;
+}
+
+// Writes N rows of a thread, key[k] and carried value val[k], to output
+// positions pos[k] (k with bit k of `live`): one column at a time, every load
+// of a gathered column issued before its stores.
+template <int N, typename V>
+__device__ __forceinline__ void emit_rows(const PassParams& p, const uint64_t (&key)[N], const V (&val)[N],
+                                          const uint32_t (&pos)[N], uint32_t live) {
+  int64_t raw[N];
+  for (int j = 0; j < p.K.nkeys; j++) {
+    const KeyField& kf = p.K.k[j];
+    const int vb = p.dec_vbits[j], vs = p.dec_vshift[j] & 63, fs = p.dec_fshift[j];
+    const uint64_t vmask = vb == 0 ? 0 : (vb >= 64 ? ~0ull : ((1ull << vb) - 1));
+    // order image = field + umin, complemented for DESC; an integer's value is
+    // its image with the sign bit flipped, that is 2^63 added; -f = ~f + 1
+    const uint64_t neg = kf.desc ? ~0ull : 0ull;
+    const uint64_t base = (kf.umin ^ neg) - neg - (kf.desc ? 1 : 0);
+    uint32_t nulls = 0;
+    if (kf.col.type == GHB_INT) {
+      const uint32_t m32 = (uint32_t)vmask, n32 = (uint32_t)neg, b32 = (uint32_t)base - n32;
+#pragma unroll
+      for (int k = 0; k < N; k++) raw[k] = (int32_t)((((uint32_t)(key[k] >> vs) & m32) ^ n32) + b32);
+    } else if (kf.col.type == GHB_LONG) {
+      const uint64_t b64 = base - neg + 0x8000000000000000ull;
+#pragma unroll
+      for (int k = 0; k < N; k++) raw[k] = (int64_t)((((key[k] >> vs) & vmask) ^ neg) + b64);
+    } else {
+#pragma unroll
+      for (int k = 0; k < N; k++) raw[k] = (int64_t)unflip_f64_bits((((key[k] >> vs) & vmask) ^ neg) + base - neg);
+    }
+    if (fs >= 0) {
+      const bool nf = kf.nulls_first;
+#pragma unroll
+      for (int k = 0; k < N; k++) nulls |= ((((key[k] >> fs) & 1ull) == 0) == nf ? 1u : 0u) << k;
+    }
+    put_rows<N>(p.out_keys[j], kf.col.type, raw, nulls, pos, live);
+  }
+  int64_t row[N];   // a carried payload's raw value, or the row index
+#pragma unroll
+  for (int k = 0; k < N; k++) row[k] = sizeof(V) == 4 ? (int64_t)(int32_t)val[k] : (int64_t)val[k];
+  if (!p.carry_rowid) {
+    if (p.npay == 1) {
+      const ghb_column& c = p.pay[0];
+      put_rows<N>(p.out_pay[0], c.type, row, c.null_mode == GHB_NULLS_SENTINEL ? null_bits<N>(c, row, row, live) : 0u,
+                  pos, live);
+    }
+    return;
+  }
+  if (p.out_rowid) {
+#pragma unroll
+    for (int k = 0; k < N; k++)
+      if (live >> k & 1) p.out_rowid[pos[k]] = (int32_t)row[k];
+  }
+  for (int j = 0; j < p.npay; j++) {
+    const ghb_column& c = p.pay[j];
+#pragma unroll
+    for (int k = 0; k < N; k++) raw[k] = live >> k & 1 ? ld_raw(c, row[k]) : 0;
+    put_rows<N>(p.out_pay[j], c.type, raw, null_bits<N>(c, raw, row, live), pos, live);
+  }
+}
+
+constexpr int kFinItems = 4;                         // rows a thread works on together
+constexpr int kFinTile = 2 * kSortThreads * kFinItems;   // 2048 rows
+constexpr int kFinRounds = 2;                        // further rows read to find a run's end:
+constexpr int kFinExt = 32 + kFinRounds * kSortThreads;   // 32, then 256 a round
+constexpr int kFinNet = 16;                          // longest run one thread sorts
+constexpr int kFinField = 28;                        // key bits such a sort compares
+
+__device__ __forceinline__ void word_order(uint32_t& a, uint32_t& b) {
+  const uint32_t lo = min(a, b);
+  b = max(a, b);
+  a = lo;
+}
+
+// Sorts the first N words in registers by odd-even merges (Batcher): the
+// comparators of distance K of the merges into blocks of 2 P words, then of
+// K / 2, then those of 2 P.
+template <int N, int P = 1, int K = 1>
+__device__ __forceinline__ void sort_words(uint32_t (&w)[kFinNet]) {
+#pragma unroll
+  for (int e = K % P; e + K < N; e++)
+    if ((e - K % P) % (2 * K) < K && e / (2 * P) == (e + K) / (2 * P)) word_order(w[e], w[e + K]);
+  if constexpr (K > 1) sort_words<N, P, K / 2>(w);
+  else if constexpr (2 * P < N) sort_words<N, 2 * P, 2 * P>(w);
+}
+
+// One run of len <= N rows from row a on, put in order by one thread: words
+// (field, place in the run) sorted in registers, then the rows that differ
+// only below the field by insertion.
+template <int N>
+__device__ __forceinline__ void sort_run(const uint64_t* s_key, const uint32_t* s_word, uint16_t* s_src, int a, int len,
+                                         bool partial) {
+  uint32_t w[kFinNet];
+#pragma unroll
+  for (int k = 0; k < N; k++) w[k] = k < len ? s_word[a + k] | k : 0xffffffffu;
+  sort_words<N>(w);
+  bool tie = false;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    if (k < len) s_src[a + k] = (uint16_t)(a + (w[k] & 15u));
+    if (partial && k > 0 && k < len) tie |= (w[k] ^ w[k - 1]) < 16u;
+  }
+  if (tie)
+    for (int i = 1; i < len; i++) {
+      const uint16_t x = s_src[a + i];
+      int j = i;
+      for (; j > 0 && s_key[x] < s_key[s_src[a + j - 1]]; j--) s_src[a + j] = s_src[a + j - 1];
+      s_src[a + j] = x;
+    }
+}
+
+// The rows are sorted by their keys' bits from p.shift up; a tile puts the
+// runs that start in it (equal bits from p.shift up) in order by the lower
+// bits and writes their rows, in output order.  A run of up to kFinNet rows is
+// sorted by one thread in registers; a longer one by a warp: each row's place
+// is the number of smaller keys in the run and of equal ones before it.  A run
+// whose end is not found within kFinExt rows of the tile goes to the list of
+// long runs.  Bound by instruction issue (205 per 32 rows at six rows to a
+// run; DRAM 35 %): 0.54 ms for the 60M-row (d, k) sort, which it spares four
+// passes of 0.40 ms.  Other forms measured there: every row counting the rows
+// of its run before it 1.04 ms, with 64-bit keys in shared memory 0.96; one
+// list of runs found by a thread per row 0.71.
+template <typename V>
+__global__ void __launch_bounds__(kSortThreads) sort_finish_kernel(const __grid_constant__ PassParams p) {
+  constexpr int kRows = kFinTile + kFinExt;
+  constexpr int kWords = kRows / 32;
+  constexpr int kTileWords = kFinTile / 32;
+  static_assert(kFinTile == 8 * kSortThreads && kFinTile == 2048 && kFinNet == 16, "a run's list entry");
+  constexpr int kRuns = kFinTile / 2 + 1;        // runs of two rows and more that start in a tile
+  __shared__ uint64_t s_key[kRows];
+  __shared__ uint32_t s_word[kRows];             // the key's field << 4
+  __shared__ uint16_t s_src[kRows];              // row of the tile that goes to each place
+  __shared__ uint16_t s_run[kRuns];              // (rows - 1) << 11 | first row: runs of up to 8 rows from the
+                                                 // front, of up to kFinNet from the back
+  __shared__ uint16_t s_big[kRows / kFinNet];    // first rows of longer runs
+  __shared__ uint32_t s_start[kWords + 1];       // bit i: row i starts a run
+  __shared__ uint32_t s_n[2];                    // runs in the lists: up to 8 rows | up to kFinNet << 16; longer
+  if (*(volatile int32_t*)p.dev_status == kDevTimeout) return;   // the passes left invalid rows
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int64_t t0 = (int64_t)blockIdx.x * kFinTile;
+  const int left = (int)min(p.n - t0, (int64_t)kRows);   // rows from the tile's first to the end
+  const unsigned long long* keys_in = (const unsigned long long*)p.keys_in + t0;
+  const V* vals_in = (const V*)p.vals_in + t0;
+  const uint64_t lead = ~0ull << p.shift;                // 0 < p.shift < 64
+  const int fshift = max(0, p.shift - kFinField);
+  const uint32_t fmask = (1u << min(p.shift, kFinField)) - 1u;
+  if (threadIdx.x < 2) s_n[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_start[kWords] = 0;
+  // row i of the tile: its key to shared memory, and its start flag
+  auto enter = [&](int i, uint64_t key) -> uint32_t {
+    uint64_t prev = __shfl_up_sync(0xffffffffu, key, 1);
+    if (lane == 0) prev = t0 + i > 0 && i < left ? keys_in[i - 1] : ~key;
+    const uint32_t sw = __ballot_sync(0xffffffffu, i >= left || ((prev ^ key) & lead));   // rows past the end
+                                                                                          // close the last run
+    s_key[i] = key;
+    s_word[i] = ((uint32_t)(key >> fshift) & fmask) << 4;
+    s_src[i] = (uint16_t)i;
+    if (lane == 0) s_start[i >> 5] = sw;
+    return sw;
+  };
+  for (int h = 0; h < kFinTile; h += kSortThreads * kFinItems) {
+    uint64_t x[kFinItems];
+#pragma unroll
+    for (int k = 0; k < kFinItems; k++) {
+      const int i = h + k * kSortThreads + threadIdx.x;
+      x[k] = i < left ? __ldcs(keys_in + i) : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < kFinItems; k++) enter(h + k * kSortThreads + threadIdx.x, x[k]);
+  }
+  // the rows after the tile up to the start of a run
+  if (warp == 0) enter(kFinTile + lane, kFinTile + lane < left ? keys_in[kFinTile + lane] : 0);
+  __syncthreads();
+  int rows = kFinTile + 32;                        // rows entered
+  bool closed = s_start[kTileWords] != 0;          // the last run's end is among them
+  for (int q = 0; q < kFinRounds && !closed; q++) {
+    const int i = rows + threadIdx.x;
+    closed = __syncthreads_or(enter(i, i < left ? keys_in[i] : 0) != 0);
+    rows += kSortThreads;
+  }
+  // first start after row i, `rows` if there is none
+  auto next_start = [&](int i) -> int {
+    int w = i >> 5;
+    uint32_t m = s_start[w] & (0xfffffffeu << (i & 31));
+    while (m == 0 && (w + 1) * 32 < rows) m = s_start[++w];
+    return m ? w * 32 + __ffs(m) - 1 : rows;
+  };
+  // [begin, end): the runs that start in the tile; an open one is a long run
+  int begin = kFinTile, end = 0;
+  for (int w = 0; w < kTileWords; w++)
+    if (s_start[w]) {
+      begin = w * 32 + __ffs(s_start[w]) - 1;
+      break;
+    }
+  if (begin >= min(left, kFinTile)) return;        // the whole tile belongs to an earlier tile's run
+  if (closed) {
+    end = min(left, next_start(kFinTile - 1));
+  } else {
+    for (int w = kTileWords - 1;; w--)
+      if (s_start[w]) {
+        end = w * 32 + 31 - __clz(s_start[w]);
+        break;
+      }
+    if (threadIdx.x == 0) p.long_runs[1 + atomicAdd(&p.long_runs[0], 1u)] = (uint32_t)(t0 + end);
+  }
+  // list the runs of two rows and more: eight rows a thread, from the bits of
+  // its rows and the 24 after them
+  {
+    const int r0 = 8 * threadIdx.x;
+    const int w = threadIdx.x >> 2;
+    const uint32_t win = __funnelshift_r(s_start[w], s_start[w + 1], 8 * (threadIdx.x & 3));
+    uint32_t mine = win & 0xffu;
+    if (end - r0 < 8) mine &= end > r0 ? (1u << (end - r0)) - 1u : 0u;
+    mine &= ~(win >> 1);                               // not runs of one row
+    uint32_t n = 0;                                    // runs of up to 8 rows, of up to kFinNet << 16
+    for (uint32_t m = mine; m; m &= m - 1) {
+      const int len = __ffs(win >> __ffs(m));
+      n += len == 0 || len > kFinNet ? 0u : len <= 8 ? 1u : 1u << 16;
+    }
+    uint32_t incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    uint32_t at = 0;
+    if (lane == 31) at = atomicAdd(&s_n[0], incl);
+    at = __shfl_sync(0xffffffffu, at, 31) + incl - n;
+    for (uint32_t m = mine; m; m &= m - 1) {
+      const int j = __ffs(m) - 1, len = __ffs(win >> (j + 1));
+      if (len == 0 || len > kFinNet) {
+        s_big[atomicAdd(&s_n[1], 1u)] = (uint16_t)(r0 + j);
+      } else if (len <= 8) {
+        s_run[at & 0xffffu] = (uint16_t)((len - 1) << 11 | (r0 + j));
+        at += 1;
+      } else {
+        s_run[kRuns - 1 - (at >> 16)] = (uint16_t)((len - 1) << 11 | (r0 + j));
+        at += 1u << 16;
+      }
+    }
+  }
+  __syncthreads();
+  const int n8 = s_n[0] & 0xffffu, n16 = s_n[0] >> 16, nbig = s_n[1];
+  for (int m = warp; m < nbig; m += kSortThreads / 32) {
+    const int a = s_big[m], b = next_start(a);
+    bool desc = false;
+    for (int i = a + 1 + lane; i < b; i += 32) desc |= s_key[i] < s_key[i - 1];
+    if (!__any_sync(0xffffffffu, desc)) continue;   // in order already
+    for (int i = a + lane; i < b; i += 32) {
+      const uint64_t mine = s_key[i];
+      int at = a;
+      for (int j = a; j < b; j++) at += s_key[j] < mine || (s_key[j] == mine && j < i);
+      s_src[at] = (uint16_t)i;
+    }
+  }
+  for (int r = threadIdx.x; r < n16; r += kSortThreads) {
+    const int e = s_run[kRuns - 1 - r];
+    sort_run<16>(s_key, s_word, s_src, e & 2047, (e >> 11) + 1, fshift > 0);
+  }
+  // the other way round, so that the warps without a run above go first
+  for (int r = kSortThreads - 1 - threadIdx.x; r < n8; r += kSortThreads) {
+    const int e = s_run[r], a = e & 2047, len = (e >> 11) + 1;
+    if (__any_sync(__activemask(), len > 4)) sort_run<8>(s_key, s_word, s_src, a, len, fshift > 0);
+    else sort_run<4>(s_key, s_word, s_src, a, len, fshift > 0);
+  }
+  __syncthreads();
+  for (int h = 0; h < kFinTile && h < end; h += kSortThreads * kFinItems) {
+    V val[kFinItems];
+    uint64_t x[kFinItems];
+    uint32_t pos[kFinItems], live = 0;
+#pragma unroll
+    for (int k = 0; k < kFinItems; k++) {
+      const int i = h + k * kSortThreads + threadIdx.x;
+      const bool mine = i >= begin && i < end;
+      const int src = mine ? s_src[i] : 0;
+      val[k] = mine ? vals_in[src] : (V)0;
+      x[k] = s_key[src];
+      pos[k] = (uint32_t)t0 + (uint32_t)i;
+      live |= (mine ? 1u : 0u) << k;
+    }
+    emit_rows<kFinItems, V>(p, x, val, pos, live);
+  }
+  for (int i = kFinTile + threadIdx.x; i < end; i += kSortThreads) {   // the last run's rows past the tile
+    const uint64_t x[1] = {s_key[s_src[i]]};
+    const V v[1] = {vals_in[s_src[i]]};
+    const uint32_t at[1] = {(uint32_t)t0 + (uint32_t)i};
+    emit_rows<1, V>(p, x, v, at, 1u);
+  }
+}
+
+// The long runs, one CTA each: rows already in order are written as they are;
+// else a stable LSD radix sort of the run by its lower bits, through the other
+// ping-pong buffer.
+constexpr int kLongThreads = 1024;
+
+template <typename V>
+__global__ void __launch_bounds__(kLongThreads) sort_finish_long_kernel(const __grid_constant__ PassParams p) {
+  __shared__ uint32_t s_hist[kBins], s_base[kBins];
+  __shared__ uint16_t s_wcnt[kLongThreads / 32][kBins];
+  __shared__ int64_t s_end;
+  if (*(volatile int32_t*)p.dev_status == kDevTimeout) return;
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const uint32_t count = *(volatile uint32_t*)p.long_runs;
+  for (uint32_t q = blockIdx.x; q < count; q += gridDim.x) {
+    const int64_t a = p.long_runs[1 + q];
+    uint64_t* kb[2] = {(uint64_t*)p.keys_in, p.keys_out};
+    V* vb[2] = {(V*)p.vals_in, (V*)p.vals_out};
+    if (threadIdx.x == 0) {   // the run's end: the leading bits ascend
+      const uint64_t top = kb[0][a] >> p.shift;
+      int64_t lo = a, hi = p.n;   // kb[lo] in the run, hi past it
+      while (hi - lo > 1) {
+        const int64_t m = lo + (hi - lo) / 2;
+        if (kb[0][m] >> p.shift == top) lo = m;
+        else hi = m;
+      }
+      s_end = hi;
+    }
+    __syncthreads();
+    const int64_t b = s_end;
+    bool desc = false;
+    for (int64_t i = a + 1 + threadIdx.x; i < b; i += kLongThreads) desc |= kb[0][i] < kb[0][i - 1];
+    int cur = 0;
+    if (__syncthreads_or(desc))
+      for (int sh = 0; sh < p.shift; sh += kDigitBits) {
+        const uint32_t mask = min(kBins, 1 << min(kDigitBits, p.shift - sh)) - 1;
+        for (int i = threadIdx.x; i < kBins; i += kLongThreads) s_hist[i] = 0;
+        __syncthreads();
+        for (int64_t i = a + threadIdx.x; i < b; i += kLongThreads)
+          atomicAdd(&s_hist[(uint32_t)(kb[cur][i] >> sh) & mask], 1u);
+        __syncthreads();
+        if (warp == 0) {   // exclusive offsets, eight digits a lane
+          uint32_t v[kBins / 32], sum = 0;
+#pragma unroll
+          for (int k = 0; k < kBins / 32; k++) {
+            v[k] = s_hist[lane * (kBins / 32) + k];
+            sum += v[k];
+          }
+          uint32_t incl = sum;
+          for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+          }
+          uint32_t run = incl - sum;
+#pragma unroll
+          for (int k = 0; k < kBins / 32; k++) {
+            s_base[lane * (kBins / 32) + k] = run;
+            run += v[k];
+          }
+        }
+        for (int64_t c = a; c < b; c += kLongThreads) {
+          for (int i = threadIdx.x; i < kLongThreads / 32 * kBins; i += kLongThreads) (&s_wcnt[0][0])[i] = 0;
+          __syncthreads();
+          const int64_t i = c + threadIdx.x;
+          const bool live = i < b;
+          const uint64_t x = live ? kb[cur][i] : 0;
+          const V v = live ? vb[cur][i] : (V)0;
+          const uint32_t dk = live ? (uint32_t)(x >> sh) & mask : kBins;
+          const unsigned peers = __match_any_sync(0xffffffffu, dk);
+          const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+          if (live && rank == 0) s_wcnt[warp][dk] = (uint16_t)__popc(peers);
+          __syncthreads();
+          if (threadIdx.x < kBins) {
+            uint32_t run = s_base[threadIdx.x];
+            for (int w = 0; w < kLongThreads / 32; w++) {
+              const uint32_t t = s_wcnt[w][threadIdx.x];
+              s_wcnt[w][threadIdx.x] = (uint16_t)(run - s_base[threadIdx.x]);
+              run += t;
+            }
+            s_hist[threadIdx.x] = run;
+          }
+          __syncthreads();
+          if (live) {
+            const int64_t to = a + s_base[dk] + s_wcnt[warp][dk] + rank;
+            kb[cur ^ 1][to] = x;
+            vb[cur ^ 1][to] = v;
+          }
+          __syncthreads();
+          if (threadIdx.x < kBins) s_base[threadIdx.x] = s_hist[threadIdx.x];
+          __syncthreads();
+        }
+        cur ^= 1;
+      }
+    for (int64_t i = a + threadIdx.x; i < b; i += kLongThreads) {
+      const uint64_t x[1] = {kb[cur][i]};
+      const V v[1] = {vb[cur][i]};
+      const uint32_t at[1] = {(uint32_t)i};
+      emit_rows<1, V>(p, x, v, at, 1u);
+    }
+    __syncthreads();   // s_end and the run's buffers are done with
+  }
+}
+
 // Output in input order (keys all equal, or n tiny): gathers row r to r, or
 // row perm[r] to r when a permutation is given.
 template <typename V>
@@ -699,6 +1301,9 @@ __global__ void sort_identity_kernel(PassParams p, const V* perm) {
        r += (int64_t)gridDim.x * blockDim.x)
     gather_write(p, perm ? (int64_t)perm[r] : r, r);
 }
+
+// Words of the analysis: three per key, then the sample's pair counts.
+constexpr int kStatWords = 3 * kMaxSortKeys + 9;
 
 static inline size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
@@ -710,7 +1315,8 @@ size_t sort_scratch_bytes(int64_t n) {
   b += 2 * align256((size_t)n * 8);                        // values ping-pong
   b += 2 * align256((size_t)ntiles * kBins * 4);           // look-back words of two passes
   b += align256((size_t)kMaxSeg * kMaxPasses * kBins * 4); // histograms
-  b += align256(3 * 8 * kMaxSortKeys);                     // min/max
+  b += align256(kStatWords * 8);                           // min/max, sample
+  b += align256(((size_t)n / kFinTile + 2) * 4);           // long runs
   return b + 4096;
 }
 
@@ -752,8 +1358,9 @@ static int32_t set_smem(ghb_ctx* ctx, size_t dyn) {
 template <typename V>
 static int32_t run_passes(ghb_ctx* ctx, PassParams& pp, const std::vector<Segment>& segs,
                           const std::vector<std::vector<int>>& run, const uint32_t* d_hist,
-                          uint64_t* const kb[2], void* const vbv[2], bool packed, cudaStream_t stream) {
+                          uint64_t* const kb[2], void* const vbv[2], bool packed, int shift0, cudaStream_t stream) {
   int32_t st;
+  const bool finish = shift0 > 0;   // the passes leave the lower bits to the finish
   int total = 0;
   for (auto& r : run) total += (int)r.size();
   const int64_t n = pp.n;
@@ -786,8 +1393,8 @@ static int32_t run_passes(ghb_ctx* ctx, PassParams& pp, const std::vector<Segmen
       int q = run[s][i];
       bool last = ++done == total;
       int src = i == 0 ? (have_perm ? kSrcPerm : packed ? kSrcPacked : kSrcCols) : kSrcPacked;
-      int dst = last ? (multi ? kDstGather : kDstDecode) : kDstPacked;
-      pp.shift = q * kDigitBits;
+      int dst = last && !finish ? (multi ? kDstGather : kDstDecode) : kDstPacked;
+      pp.shift = shift0 + q * kDigitBits;
       pp.hist = d_hist + ((size_t)s * kMaxPasses + q) * kBins;
       pp.keys_in = kb[cur];
       pp.vals_in = vb[cur];
@@ -801,7 +1408,44 @@ static int32_t run_passes(ghb_ctx* ctx, PassParams& pp, const std::vector<Segmen
       have_perm = true;
     }
   }
+  if (finish) {
+    pp.keys_in = kb[cur];
+    pp.vals_in = vb[cur];
+    pp.keys_out = kb[cur ^ 1];
+    pp.vals_out = vb[cur ^ 1];
+    pp.shift = shift0;
+    const int fgrid = (int)((n + kFinTile - 1) / kFinTile);
+    sort_finish_kernel<V><<<fgrid, kSortThreads, 0, stream>>>(pp);
+    GHB_LAUNCH_CHECK(ctx);
+    const int lgrid = (int)std::min<int64_t>(n / kFinTile + 1, ctx->num_sms);
+    sort_finish_long_kernel<V><<<lgrid, kLongThreads, 0, stream>>>(pp);
+    GHB_LAUNCH_CHECK(ctx);
+  }
   return GHB_OK;
+}
+
+// How many leading digits of a one-segment key of `bits` bits the passes
+// sort by, from the sample's pair counts; 0: all of them.  In units of a
+// thirtieth of a pass (14 us at 60M rows): the finish costs 38 where a last
+// pass that decodes costs 40, and each row has n * pairs / S^2 others in its
+// run, cheap while one thread sorts the run in registers (60M rows of about
+// six to a run: 0.54 ms) and dear beyond it (1M rows: the finish takes 15 us
+// at one or two rows to a run, 40 at 25, a pass 17).  Rows expected in runs of
+// more than 32 are never left to the finish.
+static int leading_digits(int bits, int64_t n, const unsigned long long* pairs, int S, int first) {
+  const int all = (bits + kDigitBits - 1) / kDigitBits;
+  int best = 0;
+  double cost = 30.0 * all + 10;
+  for (int q = first; q * kDigitBits < bits && q <= 8; q++) {
+    const double mates = (double)n * (double)pairs[q] / ((double)S * S);
+    if (mates > 32) continue;
+    const double c = 30.0 * q + 38 + 0.5 * mates + 2.0 * std::max(0.0, mates - 6);
+    if (c < cost) {
+      cost = c;
+      best = q;
+    }
+  }
+  return best;
 }
 
 int32_t sort_impl(ghb_ctx* ctx, const ghb_column* keys, const int32_t* orders,
@@ -842,13 +1486,15 @@ int32_t sort_impl(ghb_ctx* ctx, const ghb_column* keys, const int32_t* orders,
     int no = null_orders ? null_orders[j] : GHB_NULLS_DEFAULT;
     K.k[j].nulls_first = no == GHB_NULLS_FIRST || (no == GHB_NULLS_DEFAULT && !K.k[j].desc);
   }
+  // one zeroed block: the analysis, the histograms, the count of long runs
   unsigned long long* d_mm = nullptr;
-  uint32_t* d_hist = nullptr;
-  if ((st = scratch_alloc(ctx, 3 * 8 * kMaxSortKeys, (void**)&d_mm, stream))) return st;
-  if ((st = scratch_alloc(ctx, (size_t)kMaxSeg * kMaxPasses * kBins * 4, (void**)&d_hist, stream))) return st;
-  std::vector<unsigned long long> mm_init(3 * kMaxSortKeys, 0);
-  for (int j = 0; j < kMaxSortKeys; j++) mm_init[3 * j] = ~0ull;
-  GHB_CUDA_TRY(ctx, cudaMemcpyAsync(d_mm, mm_init.data(), mm_init.size() * 8, cudaMemcpyHostToDevice, stream));
+  const size_t stat_bytes = align256(kStatWords * 8), hist_bytes = (size_t)kMaxSeg * kMaxPasses * kBins * 4;
+  if ((st = scratch_alloc(ctx, stat_bytes + hist_bytes + align256(((size_t)n / kFinTile + 2) * 4), (void**)&d_mm,
+                          stream)))
+    return st;
+  uint32_t* d_hist = (uint32_t*)((char*)d_mm + stat_bytes);
+  uint32_t* d_long = d_hist + hist_bytes / 4;
+  GHB_CUDA_TRY(ctx, cudaMemsetAsync(d_mm, 0, stat_bytes + hist_bytes + 4, stream));
   int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)ctx->num_sms * 8);
   MinMaxParams mp;
   mp.K = K;
@@ -856,7 +1502,19 @@ int32_t sort_impl(ghb_ctx* ctx, const ghb_column* keys, const int32_t* orders,
   mp.out = d_mm;
   sort_minmax_kernel<<<grid, 256, 0, stream>>>(mp);
   GHB_LAUNCH_CHECK(ctx);
-  unsigned long long mm[3 * kMaxSortKeys];
+  // the fewest leading digits whose runs, were the keys spread evenly, would
+  // stay at 32 rows; a sample whose one pair stands for few rows
+  SampleParams sp;
+  sp.first = 1;
+  while (sp.first < 4 && (n >> (kDigitBits * sp.first)) > 32) sp.first++;
+  sp.S = n > (4 << 20) ? kSampleMax : 1024;
+  sp.K = K;
+  sp.n = n;
+  sp.mm = d_mm;
+  sp.pairs = d_mm + 3 * kMaxSortKeys;
+  sort_sample_kernel<<<sp.S / kSampleRows, 256, 0, stream>>>(sp);
+  GHB_LAUNCH_CHECK(ctx);
+  unsigned long long mm[kStatWords];
   GHB_CUDA_TRY(ctx, cudaMemcpyAsync(mm, d_mm, sizeof(mm), cudaMemcpyDeviceToHost, stream));
   GHB_CUDA_TRY(ctx, cudaStreamSynchronize(stream));
 
@@ -879,9 +1537,8 @@ int32_t sort_impl(ghb_ctx* ctx, const ghb_column* keys, const int32_t* orders,
   };
   for (int j = nkeys - 1; j >= 0; j--) {
     KeyField& f = K.k[j];
-    bool anyval = mm[3 * j] <= mm[3 * j + 1];
-    f.umin = anyval ? mm[3 * j] : 0;
-    uint64_t range = anyval ? mm[3 * j + 1] - mm[3 * j] : 0;
+    uint64_t range;
+    key_range(mm + 3 * j, &f.umin, &range);
     f.vbits = range == 0 ? 0 : 64 - __builtin_clzll(range);
     f.has_null = mm[3 * j + 2] ? 1 : 0;
     add_sub(j, 0, f.vbits);
@@ -902,13 +1559,16 @@ int32_t sort_impl(ghb_ctx* ctx, const ghb_column* keys, const int32_t* orders,
     if ((st = scratch_alloc(ctx, (size_t)n * vw, &vb[i], stream))) return st;
   }
 
-  // histograms of every segment, one read each, then one sync; a
-  // one-segment key is packed on the way
-  GHB_CUDA_TRY(ctx, cudaMemsetAsync(d_hist, 0, segs.size() * kMaxPasses * kBins * 4, stream));
+  // the leading digits alone, when the finish is to sort the rest
+  const int top = multi ? 0 : leading_digits(segs[0].bits, n, mm + 3 * kMaxSortKeys, sp.S, sp.first);
+  const int shift0 = top ? segs[0].bits - top * kDigitBits : 0;
+  // histograms of every segment, one read each; a one-segment key is packed
+  // on the way
   for (size_t s = 0; s < segs.size(); s++) {
-    int np = (segs[s].bits + kDigitBits - 1) / kDigitBits;
+    int np = top ? top : (segs[s].bits + kDigitBits - 1) / kDigitBits;
     if (np == 0) continue;
     HistParams hp;
+    hp.shift0 = shift0;
     hp.K = K;
     hp.seg = segs[s];
     hp.n = n;
@@ -942,17 +1602,22 @@ int32_t sort_impl(ghb_ctx* ctx, const ghb_column* keys, const int32_t* orders,
     sort_hist_kernel<<<std::min(grid, ctx->num_sms * 8), 256, 0, stream>>>(hp);
     GHB_LAUNCH_CHECK(ctx);
   }
-  std::vector<uint32_t> hist((size_t)segs.size() * kMaxPasses * kBins, 0);
-  GHB_CUDA_TRY(ctx, cudaMemcpyAsync(hist.data(), d_hist, hist.size() * 4, cudaMemcpyDeviceToHost, stream));
-  GHB_CUDA_TRY(ctx, cudaStreamSynchronize(stream));
   std::vector<std::vector<int>> run(segs.size());
-  for (size_t s = 0; s < segs.size(); s++) {
-    int np = (segs[s].bits + kDigitBits - 1) / kDigitBits;
-    for (int q = 0; q < np; q++) {
-      bool trivial = false;
-      for (int b = 0; b < kBins; b++)
-        if (hist[((size_t)s * kMaxPasses + q) * kBins + b] == (uint32_t)n) trivial = true;
-      if (!trivial) run[s].push_back(q);
+  if (top) {
+    for (int q = 0; q < top; q++) run[0].push_back(q);
+  } else {
+    // every digit is sorted by: the host skips passes whose digit is constant
+    std::vector<uint32_t> hist((size_t)segs.size() * kMaxPasses * kBins, 0);
+    GHB_CUDA_TRY(ctx, cudaMemcpyAsync(hist.data(), d_hist, hist.size() * 4, cudaMemcpyDeviceToHost, stream));
+    GHB_CUDA_TRY(ctx, cudaStreamSynchronize(stream));
+    for (size_t s = 0; s < segs.size(); s++) {
+      int np = (segs[s].bits + kDigitBits - 1) / kDigitBits;
+      for (int q = 0; q < np; q++) {
+        bool trivial = false;
+        for (int b = 0; b < kBins; b++)
+          if (hist[((size_t)s * kMaxPasses + q) * kBins + b] == (uint32_t)n) trivial = true;
+        if (!trivial) run[s].push_back(q);
+      }
     }
   }
 
@@ -985,9 +1650,10 @@ int32_t sort_impl(ghb_ctx* ctx, const ghb_column* keys, const int32_t* orders,
   pp.counters = ctx->d_counters + 2;
   pp.dev_status = ctx->d_status;
   pp.spin_limit = ctx->spin_limit;
+  pp.long_runs = d_long;
   const bool packed = !multi;
-  if (wide) return run_passes<uint64_t>(ctx, pp, segs, run, d_hist, kb, vb, packed, stream);
-  return run_passes<uint32_t>(ctx, pp, segs, run, d_hist, kb, vb, packed, stream);
+  if (wide) return run_passes<uint64_t>(ctx, pp, segs, run, d_hist, kb, vb, packed, shift0, stream);
+  return run_passes<uint32_t>(ctx, pp, segs, run, d_hist, kb, vb, packed, shift0, stream);
 }
 
 // ---------------------------------------------------------------- STRING keys
