@@ -324,24 +324,23 @@ __device__ __forceinline__ uint64_t lb_load(const uint64_t* p) {
   return v;
 }
 
-// Exclusive prefix of tile `tile` given its own `count`.  Called by one warp
-// (all 32 lanes).  Publishes the tile's aggregate, walks back over earlier
-// tiles 32 at a time, then publishes the inclusive prefix.  The words carry
-// only counts (no tile reads another tile's output), so relaxed stores and
-// loads suffice and no fence is needed.  Every wait is bounded: after
-// `spin_limit` polls that find an earlier tile not ready it raises
-// GHB_ERR_TIMEOUT and returns 0 (the results of that launch are then invalid
-// and the host is told; every output position stays below the true one, so
-// no write leaves its buffer).
-__device__ __forceinline__ uint64_t lookback_exclusive(uint64_t* status_arr, uint32_t epoch,
-                                                       int64_t tile, uint64_t count,
-                                                       int32_t* dev_status, int spin_limit) {
+// Publishes tile `tile`'s own count (one thread): tile 0's is its prefix.
+__device__ __forceinline__ void lookback_publish(uint64_t* status_arr, uint32_t epoch, int64_t tile, uint64_t count) {
+  lb_store(&status_arr[tile], lb_pack(epoch, tile == 0 ? kFlagPrefix : kFlagAgg, count));
+}
+
+// Exclusive prefix of tile `tile` given its own, already published `count`.
+// Called by one warp (all 32 lanes): walks back over earlier tiles 32 at a
+// time, then publishes the inclusive prefix.  The words carry only counts (no
+// tile reads another tile's output), so relaxed stores and loads suffice and
+// no fence is needed.  Every wait is bounded: after `spin_limit` polls that
+// find an earlier tile not ready it raises GHB_ERR_TIMEOUT and returns 0 (the
+// results of that launch are then invalid and the host is told; every output
+// position stays below the true one, so no write leaves its buffer).
+__device__ __forceinline__ uint64_t lookback_walk(uint64_t* status_arr, uint32_t epoch, int64_t tile, uint64_t count,
+                                                  int32_t* dev_status, int spin_limit) {
   const int lane = threadIdx.x & 31;
-  if (tile == 0) {
-    if (lane == 0) lb_store(&status_arr[0], lb_pack(epoch, kFlagPrefix, count));
-    return 0;
-  }
-  if (lane == 0) lb_store(&status_arr[tile], lb_pack(epoch, kFlagAgg, count));
+  if (tile == 0) return 0;
   uint64_t exclusive = 0;
   int64_t base = tile - 1;  // highest tile index the warp examines this round
   int spins = 0;
@@ -384,6 +383,13 @@ __device__ __forceinline__ uint64_t lookback_exclusive(uint64_t* status_arr, uin
   }
   if (lane == 0) lb_store(&status_arr[tile], lb_pack(epoch, kFlagPrefix, exclusive + count));
   return exclusive;
+}
+
+// Both: publishes the tile's count and returns its exclusive prefix.
+__device__ __forceinline__ uint64_t lookback_exclusive(uint64_t* status_arr, uint32_t epoch, int64_t tile,
+                                                       uint64_t count, int32_t* dev_status, int spin_limit) {
+  if ((threadIdx.x & 31) == 0) lookback_publish(status_arr, epoch, tile, count);
+  return lookback_walk(status_arr, epoch, tile, count, dev_status, spin_limit);
 }
 
 // Tiles are claimed in launch order from a global counter, so a tile's
