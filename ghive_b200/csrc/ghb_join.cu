@@ -157,6 +157,28 @@ __global__ void __launch_bounds__(256) join_key_range_kernel(ghb_column key, uns
   }
 }
 
+// Zeroes what the chosen layout reads before a build row fills it: a direct
+// table's counts and chain heads of the key range, or the hashed table's keys,
+// counts and chain heads (the payload words are read only in filled slots).
+// 1.5M dense keys: 6 us, where clearing every allocated slot cost 20.
+__global__ void __launch_bounds__(256) join_clear_kernel(BuildParams p) {
+  const JoinLayout L = join_layout(p.stats, p.key.n, p.slots);
+  const int64_t n = L.direct ? (L.drange + 3) / 4 : (p.side + 1);   // groups of four slots
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    uint4* m = (uint4*)(p.meta + i * 4);
+    m[0] = zero;
+    m[1] = zero;
+    *(uint4*)(p.chain_p1 + i * 4) = zero;
+    if (!L.direct) {
+      uint4* k = (uint4*)(p.kimg + i * 4);
+      k[0] = zero;
+      k[1] = zero;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(256) join_build_kernel(BuildParams p) {
   const JoinLayout L = join_layout(p.stats, p.key.n, p.slots);
   unsigned long long stored = 0, maxdup = 0;
@@ -257,6 +279,8 @@ struct ProbeParams {
   int32_t* status;
   int64_t build_rows;      // with slots: the table's layout (join_layout of stats)
   int64_t slots;
+  int32_t dup_bit;         // set in slot_of_row where the key has several build rows; 0: the slots
+                           // leave no bit free
 };
 
 // Output rows a probe row produces, from its slot's count (0 = no match).
@@ -342,7 +366,8 @@ __global__ void __launch_bounds__(TH) join_count_direct_kernel(ProbeParams p) {
     for (int k = 0; k < IT; k++) {
       const int off = woff + k * 32;
       if (off < left) {
-        if (keep_slots) p.slot_of_row[cbase + off] = cnt[k] > 0 ? (int32_t)d[k] : -1;
+        if (keep_slots)
+          p.slot_of_row[cbase + off] = cnt[k] > 0 ? (int32_t)d[k] | (cnt[k] > 1 ? p.dup_bit : 0) : -1;
         m_sum += (uint64_t)out_rows_of(p.join_type, unique ? (cnt[k] > 0 ? 1 : 0) : cnt[k]);
       }
     }
@@ -426,7 +451,7 @@ __global__ void __launch_bounds__(TH, TH == 512 ? 2 : TH == 256 ? 4 : 1) join_co
         }
       }
       if (off < left) {
-        p.slot_of_row[row] = slot;
+        p.slot_of_row[row] = count > 1 ? slot | p.dup_bit : slot;
         m_sum += (uint64_t)out_rows_of(p.join_type, count);
       }
     }
@@ -516,20 +541,6 @@ __global__ void __launch_bounds__(1024) join_scan_kernel(int64_t* counts, int64_
   if (t == 1023) *d_total = s_part[1023];
 }
 
-__device__ __forceinline__ void put_word(const ghb_out_column& o, int64_t pos, int type, int64_t raw,
-                                         bool null) {
-  if (null) {
-    if (type == GHB_INT) __stcs((int*)o.data + pos, INT32_MAX);
-    else if (type == GHB_LONG) __stcs((long long*)o.data + pos, (long long)INT64_MAX);
-    else __stcs((long long*)o.data + pos, 0x7ff8000000000000ll);
-  } else if (type == GHB_INT) {
-    __stcs((int*)o.data + pos, (int)raw);
-  } else {
-    __stcs((long long*)o.data + pos, (long long)raw);
-  }
-  if (o.is_null) o.is_null[pos] = null ? 1 : 0;
-}
-
 // The payload descriptors and output pointers of a probe, copied to shared
 // memory once per CTA for the general emit path below.
 struct EmitDesc {
@@ -540,7 +551,7 @@ struct EmitDesc {
   int32_t* out_prow;
   int32_t* out_brow;
   int32_t prow_base;
-  int32_t nbp, npp, n_inline;
+  int32_t nbp, npp;
 };
 
 __device__ __forceinline__ void load_emit_desc(const ProbeParams& p, EmitDesc* d) {
@@ -557,78 +568,82 @@ __device__ __forceinline__ void load_emit_desc(const ProbeParams& p, EmitDesc* d
     d->prow_base = p.prow_base;
     d->nbp = p.nbp;
     d->npp = p.npp;
-    d->n_inline = p.n_inline;
   }
   __syncthreads();
 }
 
-// One output row: probe row `prow`, build row `brow` (-1 for an outer miss /
-// semi), with the first-row payload words `w0`, `w1` when `inl` is set.  Out
-// of line, reading its descriptors from shared memory: the write kernel's hot
-// path is emit_lean, and inlined copies of this general loop would crowd its
-// registers.
-__device__ __noinline__ void emit_row(const EmitDesc* d, int64_t pos, int64_t prow, int32_t brow, bool inl,
-                                      unsigned long long w0, unsigned long long w1) {
-  if (d->out_prow) __stcs(d->out_prow + pos, (int)prow + d->prow_base);
-  if (d->out_brow) __stcs(d->out_brow + pos, brow);
-  for (int j = 0; j < d->nbp; j++) {
-    const ghb_column& c = d->bpay[j];
-    if (brow < 0) {
-      put_word(d->obp[j], pos, c.type, 0, true);
-      continue;
+// Writes raw[k] (NULL: bit k of `nulls`) to row base + pos[k], k with bit k of
+// `live`.
+template <int N>
+__device__ __forceinline__ void put_words(const ghb_out_column& o, int type, const int64_t (&raw)[N], uint32_t nulls,
+                                          int64_t base, const int64_t (&pos)[N], uint32_t live) {
+  if (type == GHB_INT) {
+    int* dst = (int*)o.data + base;
+#pragma unroll
+    for (int k = 0; k < N; k++)
+      if (live >> k & 1) __stcs(dst + pos[k], nulls >> k & 1 ? INT32_MAX : (int)raw[k]);
+  } else {
+    const long long none = type == GHB_LONG ? (long long)INT64_MAX : 0x7ff8000000000000ll;
+    long long* dst = (long long*)o.data + base;
+#pragma unroll
+    for (int k = 0; k < N; k++)
+      if (live >> k & 1) __stcs(dst + pos[k], nulls >> k & 1 ? none : (long long)raw[k]);
+  }
+  if (o.is_null) {
+    uint8_t* dst = o.is_null + base;
+#pragma unroll
+    for (int k = 0; k < N; k++)
+      if (live >> k & 1) dst[pos[k]] = nulls >> k & 1;
+  }
+}
+
+// Writes IT output rows of a thread (k with bit k of `live`) at wpos + pos[k]:
+// probe row row0 + 32 k with build row brow[k] (bit k of `hit`; else an outer
+// miss or a semi join's row), whose inline payload words are w[k] when INL.
+// One column at a time, its loads issued before its stores.
+template <int IT, bool INL>
+__device__ __forceinline__ void emit_rows(const EmitDesc& d, int n_inline, uint32_t live, uint32_t hit, int64_t wpos,
+                                          const int64_t (&pos)[IT], int64_t row0, const int32_t (&brow)[IT],
+                                          const ulonglong2 (&w)[IT]) {
+  int64_t raw[IT];
+  if (d.out_prow) {
+#pragma unroll
+    for (int k = 0; k < IT; k++)
+      if (live >> k & 1) __stcs(d.out_prow + wpos + pos[k], (int)row0 + k * 32 + d.prow_base);
+  }
+  if (d.out_brow) {
+#pragma unroll
+    for (int k = 0; k < IT; k++)
+      if (live >> k & 1) __stcs(d.out_brow + wpos + pos[k], hit >> k & 1 ? brow[k] : -1);
+  }
+  for (int j = 0; j < d.nbp; j++) {
+    const ghb_column& col = d.bpay[j];
+    if (INL && j < n_inline) {   // not a BYTEMAP column
+#pragma unroll
+      for (int k = 0; k < IT; k++) raw[k] = (int64_t)(j == 0 ? w[k].x : w[k].y);
+    } else {
+#pragma unroll
+      for (int k = 0; k < IT; k++) raw[k] = hit >> k & 1 ? ld_raw(col, brow[k]) : 0;
     }
-    int64_t raw = (inl && j < d->n_inline) ? (int64_t)(j == 0 ? w0 : w1) : ld_raw(c, brow);
-    bool null = c.null_mode != GHB_NULLS_NONE && raw_is_null(c, raw, brow);
-    put_word(d->obp[j], pos, c.type, raw, null);
-  }
-  for (int j = 0; j < d->npp; j++) {
-    const ghb_column& c = d->ppay[j];
-    int64_t raw = ld_raw(c, prow);
-    put_word(d->opp[j], pos, c.type, raw, c.null_mode != GHB_NULLS_NONE && raw_is_null(c, raw, prow));
-  }
-}
-
-// The lean case (INNER, no probe payloads, at most two build payloads, all
-// inline and non-NULL): the output descriptors are read once into registers
-// and a row is a few stores.  Constant indices keep the descriptors in the
-// parameter space; the general emit_row loops over them with a run-time
-// index.
-struct LeanOut {
-  int32_t* prow;
-  int32_t* brow;
-  int32_t prow_base;
-  void* data[kInline];
-  uint8_t* nul[kInline];
-  bool is_int[kInline];
-  int nbp;
-};
-
-__device__ __forceinline__ LeanOut lean_out(const ProbeParams& p) {
-  LeanOut o;
-  o.prow = p.out_prow;
-  o.brow = p.out_brow;
-  o.prow_base = p.prow_base;
-  o.nbp = p.nbp;
+    uint32_t nulls = live & ~hit;
+    if (col.null_mode != GHB_NULLS_NONE) {
 #pragma unroll
-  for (int j = 0; j < kInline; j++) {
-    o.data[j] = p.obp[j].data;
-    o.nul[j] = p.obp[j].is_null;
-    o.is_int[j] = p.bpay[j].type == GHB_INT;
+      for (int k = 0; k < IT; k++)
+        if (hit >> k & 1) nulls |= (raw_is_null(col, raw[k], brow[k]) ? 1u : 0u) << k;
+    }
+    put_words<IT>(d.obp[j], col.type, raw, nulls, wpos, pos, live);
   }
-  return o;
-}
-
-__device__ __forceinline__ void emit_lean(const LeanOut& o, int64_t pos, int64_t prow, int32_t brow,
-                                          unsigned long long w0, unsigned long long w1) {
-  if (o.prow) __stcs(o.prow + pos, (int)prow + o.prow_base);
-  if (o.brow) __stcs(o.brow + pos, brow);
+  for (int j = 0; j < d.npp; j++) {
+    const ghb_column& col = d.ppay[j];
 #pragma unroll
-  for (int j = 0; j < kInline; j++) {
-    if (j >= o.nbp) break;
-    const unsigned long long w = j == 0 ? w0 : w1;
-    if (o.is_int[j]) __stcs((int*)o.data[j] + pos, (int)w);
-    else __stcs((unsigned long long*)o.data[j] + pos, w);
-    if (o.nul[j]) o.nul[j][pos] = 0;
+    for (int k = 0; k < IT; k++) raw[k] = live >> k & 1 ? ld_raw(col, row0 + k * 32) : 0;
+    uint32_t nulls = 0;
+    if (col.null_mode != GHB_NULLS_NONE) {
+#pragma unroll
+      for (int k = 0; k < IT; k++)
+        if (live >> k & 1) nulls |= (raw_is_null(col, raw[k], row0 + k * 32) ? 1u : 0u) << k;
+    }
+    put_words<IT>(d.opp[j], col.type, raw, nulls, wpos, pos, live);
   }
 }
 
@@ -716,94 +731,119 @@ __global__ void __launch_bounds__(TH) join_write_lean_kernel(ProbeParams p) {
   }
 }
 
+// The write pass of every other join: any type, payloads and NULLs, duplicated
+// build keys.  A warp's rows are written one output column at a time, the
+// loads of a column issued before its stores; the further build rows of
+// duplicated keys follow their chains, a thread's rows together.  A LEFT OUTER
+// probe of 8M rows over 400k spread keys (one in ten twice), one probe and two
+// build payloads with NULL maps: 315 us when each row was written by an
+// out-of-line loop over the columns, 179 at three CTAs per SM, 168 at four (64
+// registers), 149 with the rows of a unique key told by a bit of the slot
+// instead of a load of their count; five CTAs 192.  Bound by the latency and the
+// requests of its gathers (DRAM 19 %).  One kernel that keeps a claimed range's
+// slots in shared memory, looks back a range later and writes measured slower,
+// here (449 us against 84 + 179 for the two passes) and for the lean write
+// pass on 60M rows (634-687 us against 90 + 16 + 455): the barriers, claims and
+// look-backs of a range cost more than reading the keys again.
 template <int TH, int IT>
-__global__ void __launch_bounds__(TH) join_write_kernel(ProbeParams p) {
-  constexpr int kJThreads = TH, kJItems = IT;
+__global__ void __launch_bounds__(TH, 1024 / TH) join_write_kernel(const __grid_constant__ ProbeParams p) {
   static_assert(TH * IT == kChunk, "a CTA iteration covers one chunk");
   if (p.lean && p.out_brow == nullptr && p.stats[1] <= 1) return;   // join_write_lean_kernel's case
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const bool unique = p.stats[1] <= 1;
-  // the row's (first row, count) is needed for duplicates and build row ids
-  const bool need_meta = !unique || p.out_brow != nullptr || !p.lean;
-  const LeanOut lo = lean_out(p);
+  // the first build row itself is read or written
+  const bool need_first = p.out_brow != nullptr || p.nbp > p.n_inline;
   __shared__ EmitDesc s_desc;
   load_emit_desc(p, &s_desc);
   // the next chunk's slots load while this chunk gathers and writes
-  int32_t next_s[kJItems];
+  int32_t next_s[IT];
 #pragma unroll
-  for (int k = 0; k < kJItems; k++) {
-    const int64_t row = (int64_t)blockIdx.x * kChunk + (int64_t)warp * (32 * kJItems) + k * 32 + lane;
-    next_s[k] = row < p.n ? __ldcs(p.slot_of_row + row) : -1;
+  for (int k = 0; k < IT; k++) {
+    const int64_t row = (int64_t)blockIdx.x * kChunk + (int64_t)warp * (32 * IT) + k * 32 + lane;
+    next_s[k] = row < p.n ? __ldcs(p.slot_of_row + row) : -2;
   }
   for (int64_t c = blockIdx.x; c < p.nchunks; c += gridDim.x) {
-    const int64_t wbase = c * kChunk + (int64_t)warp * (32 * kJItems);
-    int32_t s[kJItems];
+    const int64_t row0 = c * kChunk + (int64_t)warp * (32 * IT) + lane;
+    int32_t slot[IT], mult[IT], first[IT];   // slot: -1 no match, -2 past the end
+    bool dup[IT];                            // the key may have several build rows
+    ulonglong2 w[IT];
 #pragma unroll
-    for (int k = 0; k < kJItems; k++) {
-      s[k] = next_s[k];
-      const int64_t nrow = wbase + (int64_t)gridDim.x * kChunk + k * 32 + lane;
-      next_s[k] = nrow < p.n ? __ldcs(p.slot_of_row + nrow) : -1;
+    for (int k = 0; k < IT; k++) {
+      slot[k] = next_s[k];
+      dup[k] = slot[k] >= 0 && (p.dup_bit == 0 || (slot[k] & p.dup_bit));
+      if (slot[k] >= 0) slot[k] &= ~p.dup_bit;
+      const int64_t nrow = row0 + (int64_t)gridDim.x * kChunk + k * 32;
+      next_s[k] = nrow < p.n ? __ldcs(p.slot_of_row + nrow) : -2;
     }
-    ulonglong2 w[kJItems];
-    int32_t first[kJItems], cnt[kJItems];
 #pragma unroll
-    for (int k = 0; k < kJItems; k++) {
+    for (int k = 0; k < IT; k++) {
       first[k] = 0;
-      cnt[k] = s[k] >= 0 ? 1 : 0;
-      if (s[k] >= 0) {
-        if (p.nbp > 0) w[k] = p.payw[s[k]];
-        if (need_meta) {
-          const int2 m = p.meta[s[k]];
+      mult[k] = slot[k] >= 0 ? 1 : 0;
+      w[k] = make_ulonglong2(0, 0);
+      if (slot[k] >= 0) {
+        if (p.nbp > 0) w[k] = p.payw[slot[k]];
+        if (need_first || (!unique && dup[k])) {
+          const int2 m = p.meta[slot[k]];
           first[k] = m.x;
-          cnt[k] = m.y;
+          mult[k] = m.y;
         }
       }
     }
-    int32_t mult[kJItems];
-    uint32_t excl[kJItems];
-    uint32_t running = 0;
+    int64_t pos[IT];              // from the warp's offset on
+    int64_t running = 0;
 #pragma unroll
-    for (int k = 0; k < kJItems; k++) {
-      int64_t row = wbase + k * 32 + lane;
-      int32_t m = row < p.n ? out_rows_of(p.join_type, cnt[k]) : 0;
-      mult[k] = m;
-      uint32_t incl;
-      if (__all_sync(0xffffffffu, m <= 1)) {
-        unsigned bal = __ballot_sync(0xffffffffu, m == 1);
+    for (int k = 0; k < IT; k++) {
+      if (slot[k] != -2) mult[k] = out_rows_of(p.join_type, mult[k]);
+      uint32_t incl, total;
+      if (__all_sync(0xffffffffu, mult[k] <= 1)) {
+        const unsigned bal = __ballot_sync(0xffffffffu, mult[k] == 1);
         incl = __popc(bal & ((2u << lane) - 1u));
+        total = __popc(bal);
       } else {
-        incl = (uint32_t)m;
+        incl = (uint32_t)mult[k];
+#pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-          uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+          const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
           if (lane >= o) incl += t;
         }
+        total = __shfl_sync(0xffffffffu, incl, 31);
       }
-      excl[k] = running + incl - (uint32_t)m;
-      running += __shfl_sync(0xffffffffu, incl, 31);
+      pos[k] = running + incl - (uint32_t)mult[k];
+      running += total;
     }
-    const int64_t wpos = p.chunk_count[c * (kJThreads / 32) + warp];   // this warp's offset
+    const int64_t wpos = p.chunk_count[c * (TH / 32) + warp];   // this warp's offset
+    uint32_t live = 0, hit = 0;   // bit k: row k has output, and a build row
 #pragma unroll
-    for (int k = 0; k < kJItems; k++) {
-      if (mult[k] == 0) continue;
-      int64_t row = wbase + k * 32 + lane;
-      int64_t pos = wpos + excl[k];
-      if (pos + mult[k] > p.cap) {
-        raise_status(p.status, kDevCapacity);
-        continue;
+    for (int k = 0; k < IT; k++) {
+      if (mult[k] > 0) {
+        if (wpos + pos[k] + mult[k] <= p.cap) live |= 1u << k;
+        else raise_status(p.status, kDevCapacity);
       }
-      if (s[k] < 0 || p.join_type == GHB_LEFT_SEMI_JOIN) {
-        emit_row(&s_desc, pos, row, -1, false, 0, 0);
-        continue;
-      }
-      if (p.lean) emit_lean(lo, pos, row, first[k] - 1, p.nbp > 0 ? w[k].x : 0, p.nbp > 0 ? w[k].y : 0);
-      else emit_row(&s_desc, pos, row, first[k] - 1, true, p.nbp > 0 ? w[k].x : 0, p.nbp > 0 ? w[k].y : 0);
-      if (mult[k] > 1) {
-        int32_t b = p.chain_p1[s[k]] - 1;
-        for (int j = 1; j < mult[k]; j++) {
-          emit_row(&s_desc, pos + j, row, b, false, 0, 0);
-          if (j + 1 < mult[k]) b = p.next_p1[b] - 1;
-        }
+      if (slot[k] >= 0 && p.join_type != GHB_LEFT_SEMI_JOIN) hit |= 1u << k;
+    }
+    hit &= live;
+#pragma unroll
+    for (int k = 0; k < IT; k++) first[k]--;   // the build row
+    emit_rows<IT, true>(s_desc, p.n_inline, live, hit, wpos, pos, row0, first, w);
+    if (unique) continue;
+    // the further build rows of the threads' keys, a row of each chain a round
+    uint32_t more = 0;
+#pragma unroll
+    for (int k = 0; k < IT; k++) {
+      if (!(hit >> k & 1) || mult[k] <= 1) continue;
+      more |= 1u << k;
+      first[k] = p.chain_p1[slot[k]] - 1;
+    }
+    for (int j = 1; more; j++) {
+#pragma unroll
+      for (int k = 0; k < IT; k++) pos[k]++;
+      emit_rows<IT, false>(s_desc, p.n_inline, more, more, wpos, pos, row0, first, w);
+#pragma unroll
+      for (int k = 0; k < IT; k++) {
+        if (!(more >> k & 1)) continue;
+        if (j + 1 < mult[k]) first[k] = p.next_p1[first[k]] - 1;
+        else more &= ~(1u << k);
       }
     }
   }
@@ -878,11 +918,11 @@ int32_t join_build_impl(ghb_ctx* ctx, const ghb_column* build_key, const ghb_col
   t->chain = (int32_t*)((char*)t->alloc + bucket_bytes);
   t->next = (int32_t*)((char*)t->alloc + bucket_bytes + chain_bytes);
   t->d_stats = (unsigned long long*)((char*)t->alloc + bucket_bytes + chain_bytes + next_bytes);
-  // keys, counts and chain heads start at zero; the payload words are read
-  // only in slots a build row filled, so they are not cleared
-  if (cudaMemsetAsync(t->alloc, 0, key_bytes + meta_bytes, stream) != cudaSuccess ||
-      cudaMemsetAsync(t->chain, 0, chain_bytes, stream) != cudaSuccess ||
-      cudaMemsetAsync(t->d_stats, 0, 256, stream) != cudaSuccess) {
+  // join_clear_kernel zeroes the table's arrays; without a build row nothing
+  // chooses a layout, and the hashed one's are cleared here
+  if (cudaMemsetAsync(t->d_stats, 0, 256, stream) != cudaSuccess ||
+      (build_key->n == 0 && (cudaMemsetAsync(t->alloc, 0, key_bytes + meta_bytes, stream) != cudaSuccess ||
+                             cudaMemsetAsync(t->chain, 0, chain_bytes, stream) != cudaSuccess))) {
     cudaFreeAsync(t->alloc, stream);
     delete t;
     return set_error(ctx, GHB_ERR_CUDA, "memset of the join table failed");
@@ -906,6 +946,9 @@ int32_t join_build_impl(ghb_ctx* ctx, const ghb_column* build_key, const ghb_col
   if (build_key->n > 0) {
     int grid = (int)std::min<int64_t>((build_key->n + 255) / 256, (int64_t)ctx->num_sms * 8);
     join_key_range_kernel<<<grid, 256, 0, stream>>>(*build_key, t->d_stats);
+    ctx->launches++;
+    const int cgrid = (int)std::min<int64_t>((nb + 256) / 256, (int64_t)ctx->num_sms * 8);
+    join_clear_kernel<<<cgrid, 256, 0, stream>>>(p);
     ctx->launches++;
     join_build_kernel<<<grid, 256, 0, stream>>>(p);
     ctx->launches++;
@@ -1055,6 +1098,7 @@ int32_t join_probe_impl(ghb_ctx* ctx, const ghb_join_table* t, const ghb_column*
   else if (threads == 512) { GHB_COUNT(512, 2); }
   else { GHB_COUNT(256, 4); }
 #undef GHB_COUNT
+  p.dup_bit = t->slots + 4 <= (1ll << 30) ? 1 << 30 : 0;
   int per_sm = 0;
   GHB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, count_kernel, threads, 0));
   int grid = (int)std::min<int64_t>(p.nchunks, (int64_t)ctx->num_sms * std::max(1, per_sm));
