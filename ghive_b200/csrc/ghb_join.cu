@@ -648,17 +648,25 @@ __device__ __forceinline__ void emit_rows(const EmitDesc& d, int n_inline, uint3
 }
 
 // The write pass of an INNER join on unique build keys whose output is the
-// probe row and at most two inline, non-NULL build payloads (p.lean, no
-// build row ids): a row's output is its slot's two payload words or nothing,
-// so a thread keeps only slots and words and many CTAs fit on an SM.  It runs
-// beside the general write pass; the build's statistics (unique keys) choose
-// which of the two does the work and the other returns at once.
-template <int TH, int IT>
-__global__ void __launch_bounds__(TH) join_write_lean_kernel(ProbeParams p) {
-  static_assert(TH * IT == kChunk, "a CTA iteration covers one chunk");
+// probe row and at most two inline, non-NULL build payloads (p.lean, no build
+// row ids): a row's output is its slot's two payload words or nothing.  A warp
+// takes units of UNIT rows (the rows of one count): the keys or slots of a
+// unit are loaded together, then each 32 rows' words are gathered and stored.
+// It runs beside the general write pass; the build's statistics (unique keys)
+// choose which of the two does the work and the other returns at once.
+//
+// Bound by the SM's requests to L2, one per gathered row (57M rows of the 60M
+// probe).  432 us there at 40 warps per SM with one gather per thread in
+// flight; 487 us with four of a thread's gathers together and the next rows'
+// keys loaded ahead (47 registers, which also hold what the stores wait for);
+// two together 447-457 us, four 506; 56 or 64 warps 450 and 452; gathers that
+// do not allocate in L1 640 us.
+template <int UNIT>
+__global__ void __launch_bounds__(kJThreads, 5) join_write_lean_kernel(const __grid_constant__ ProbeParams p) {
   if (!(p.lean && p.out_brow == nullptr && p.stats[1] <= 1)) return;
+  constexpr int kIt = UNIT / 32;   // rows of a unit per lane
   const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
   // a direct table: the slot is the key's offset from the minimum, read from
   // the key itself (the count pass wrote no slots); a full one (every key of
   // the range present) needs no check of the slot
@@ -666,63 +674,53 @@ __global__ void __launch_bounds__(TH) join_write_lean_kernel(ProbeParams p) {
   const bool from_keys = L.direct;
   const bool full = from_keys && p.stats[2] == (unsigned long long)L.drange;
   const bool kint = p.pkey.type == GHB_INT;
-  const bool knull = p.pkey.null_mode != GHB_NULLS_NONE;
-  // a row's next input: its probe key (direct table) or its slot (hashed)
-  auto fetch = [&](int64_t row) -> long long {
-    if (row >= p.n) return 0;
-    if (!from_keys) return (long long)__ldcs(p.slot_of_row + row);
-    return kint ? (long long)__ldcs((const int*)p.pkey.data + row) : __ldcs((const long long*)p.pkey.data + row);
-  };
-  long long next_r[IT];
+  const int64_t nunits = (p.n + UNIT - 1) / UNIT;
+  for (int64_t u = ((int64_t)blockIdx.x * kJThreads + threadIdx.x) >> 5; u < nunits;
+       u += (int64_t)gridDim.x * (kJThreads / 32)) {
+    const int64_t row0 = u * UNIT + lane;
+    int32_t s[kIt];
+    if (!from_keys) {
 #pragma unroll
-  for (int k = 0; k < IT; k++)
-    next_r[k] = fetch((int64_t)blockIdx.x * kChunk + (int64_t)warp * (32 * IT) + k * 32 + lane);
-  for (int64_t c = blockIdx.x; c < p.nchunks; c += gridDim.x) {
-    const int64_t wbase = c * kChunk + (int64_t)warp * (32 * IT);
-    int32_t s[IT];
+      for (int k = 0; k < kIt; k++) s[k] = row0 + k * 32 < p.n ? __ldcs(p.slot_of_row + row0 + k * 32) : -1;
+    } else {
+      long long r[kIt];
 #pragma unroll
-    for (int k = 0; k < IT; k++) {
-      const int64_t row = wbase + k * 32 + lane;
-      const long long r = next_r[k];
-      next_r[k] = fetch(wbase + (int64_t)gridDim.x * kChunk + k * 32 + lane);
-      if (!from_keys) {
-        s[k] = row < p.n ? (int32_t)r : -1;
-      } else {
-        const unsigned long long d = (unsigned long long)r - (unsigned long long)L.dmin;
-        const bool hit = row < p.n && d < (unsigned long long)L.drange && !(knull && raw_is_null(p.pkey, r, row));
+      for (int k = 0; k < kIt; k++) {
+        const int64_t row = row0 + k * 32;
+        r[k] = 0;
+        if (row < p.n)
+          r[k] = kint ? (long long)__ldcs((const int*)p.pkey.data + row) : __ldcs((const long long*)p.pkey.data + row);
+      }
+#pragma unroll
+      for (int k = 0; k < kIt; k++) {
+        const int64_t row = row0 + k * 32;
+        const unsigned long long d = (unsigned long long)r[k] - (unsigned long long)L.dmin;
+        const bool hit = row < p.n && d < (unsigned long long)L.drange && !raw_is_null(p.pkey, r[k], row);
         s[k] = hit ? (int32_t)d : -1;
       }
+      if (!full) {
+#pragma unroll
+        for (int k = 0; k < kIt; k++)
+          if (s[k] >= 0 && p.meta[s[k]].y == 0) s[k] = -1;   // a hole of the key range
+      }
     }
-    if (from_keys && !full) {
+    int64_t at = p.chunk_count[u];   // this unit's offset
 #pragma unroll
-      for (int k = 0; k < IT; k++)
-        if (s[k] >= 0 && p.meta[s[k]].y == 0) s[k] = -1;   // a hole of the key range
-    }
-    ulonglong2 w[IT];
-#pragma unroll
-    for (int k = 0; k < IT; k++) w[k] = s[k] >= 0 && p.nbp > 0 ? p.payw[s[k]] : make_ulonglong2(0, 0);
-    uint32_t excl[IT];
-    uint32_t running = 0;
-#pragma unroll
-    for (int k = 0; k < IT; k++) {
+    for (int k = 0; k < kIt; k++) {
+      const ulonglong2 w = s[k] >= 0 && p.nbp > 0 ? p.payw[s[k]] : make_ulonglong2(0, 0);
       const unsigned bal = __ballot_sync(0xffffffffu, s[k] >= 0);
-      excl[k] = running + __popc(bal & ((1u << lane) - 1u));
-      running += __popc(bal);
-    }
-    const int64_t wpos = p.chunk_count[c * (TH / 32) + warp];   // this warp's offset
-#pragma unroll
-    for (int k = 0; k < IT; k++) {
+      const int64_t pos = at + __popc(bal & lt);
+      at += __popc(bal);
       if (s[k] < 0) continue;
-      const int64_t pos = wpos + excl[k];
       if (pos >= p.cap) {
         raise_status(p.status, kDevCapacity);
         continue;
       }
-      if (p.out_prow) __stcs(p.out_prow + pos, (int)(wbase + k * 32 + lane) + p.prow_base);
+      if (p.out_prow) __stcs(p.out_prow + pos, (int)row0 + k * 32 + p.prow_base);
 #pragma unroll
       for (int j = 0; j < kInline; j++) {
         if (j >= p.nbp) break;
-        const unsigned long long x = j == 0 ? w[k].x : w[k].y;
+        const unsigned long long x = j == 0 ? w.x : w.y;
         if (p.bpay[j].type == GHB_INT) __stcs((int*)p.obp[j].data + pos, (int)x);
         else __stcs((unsigned long long*)p.obp[j].data + pos, x);
         if (p.obp[j].is_null) p.obp[j].is_null[pos] = 0;
@@ -1093,7 +1091,7 @@ int32_t join_probe_impl(ghb_ctx* ctx, const ghb_join_table* t, const ghb_column*
   count_direct = kint ? (knull ? join_count_direct_kernel<TH, IT, true, true> : join_count_direct_kernel<TH, IT, true, false>) \
                       : (knull ? join_count_direct_kernel<TH, IT, false, true> : join_count_direct_kernel<TH, IT, false, false>); \
   write_kernel = join_write_kernel<TH, IT>;                                                  \
-  write_lean = join_write_lean_kernel<TH, IT>
+  write_lean = join_write_lean_kernel<32 * IT>
   if (threads == 128) { GHB_COUNT(128, 8); }
   else if (threads == 512) { GHB_COUNT(512, 2); }
   else { GHB_COUNT(256, 4); }
@@ -1115,9 +1113,9 @@ int32_t join_probe_impl(ghb_ctx* ctx, const ghb_join_table* t, const ghb_column*
   write_kernel<<<grid, threads, 0, stream>>>(p);
   GHB_LAUNCH_CHECK(ctx);
   if (p.lean && !p.out_brow) {   // the lean write pass, when the build's keys turn out unique
-    GHB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, write_lean, threads, 0));
-    grid = (int)std::min<int64_t>(p.nchunks, (int64_t)ctx->num_sms * std::max(1, per_sm));
-    write_lean<<<grid, threads, 0, stream>>>(p);
+    GHB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, write_lean, kJThreads, 0));
+    grid = (int)std::min<int64_t>((nunits * 32 + kJThreads - 1) / kJThreads, (int64_t)ctx->num_sms * std::max(1, per_sm));
+    write_lean<<<grid, kJThreads, 0, stream>>>(p);
   }
   GHB_LAUNCH_CHECK(ctx);
   return GHB_OK;
