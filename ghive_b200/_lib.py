@@ -21,6 +21,7 @@ _PROTOS = {
     "ghb_ctx_destroy": (I32, [P]),
     "ghb_last_error": (C.c_char_p, [P]),
     "ghb_sync": (I32, [P, P]),
+    "ghb_sync_count": (I32, [P, P, C.POINTER(I64), P]),
     "ghb_kernel_launches": (I64, [P]),
     "ghb_ctx_set_spin_limit": (I32, [P, I32]),
     "ghb_ctx_set_log": (I32, [P, C.c_char_p, I32, C.c_double]),

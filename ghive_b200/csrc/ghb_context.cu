@@ -9,6 +9,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <tuple>
 
 #include "ghb_ctx.hpp"
 
@@ -81,6 +82,23 @@ int32_t ensure_dyn_smem(ghb_ctx* ctx, const void* fn, size_t bytes) {
                      "kernel needs %zu bytes of dynamic shared memory, at most %d are available", bytes, limit);
   GHB_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
   done[key] = limit;
+  return GHB_OK;
+}
+
+int32_t resident_ctas(ghb_ctx* ctx, const void* fn, int threads, size_t smem, int* per_sm) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void*, int, size_t>, int> known;
+  int dev = 0;
+  GHB_CUDA_TRY(ctx, cudaGetDevice(&dev));
+  const auto key = std::make_tuple(dev, fn, threads, smem);
+  std::lock_guard<std::mutex> g(mu);
+  auto it = known.find(key);
+  if (it == known.end()) {
+    int n = 0;
+    GHB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, smem));
+    it = known.emplace(key, std::max(1, n)).first;
+  }
+  *per_sm = it->second;
   return GHB_OK;
 }
 
@@ -265,7 +283,8 @@ int32_t ghb_ctx_create(int32_t device, int64_t arena_bytes, ghb_ctx** out) {
   ctx->device = device;
   cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
   if (cudaMalloc((void**)&ctx->d_status, 64) != cudaSuccess ||
-      cudaMalloc((void**)&ctx->d_counters, 64 * sizeof(unsigned long long)) != cudaSuccess) {
+      cudaMalloc((void**)&ctx->d_counters, 64 * sizeof(unsigned long long)) != cudaSuccess ||
+      cudaHostAlloc((void**)&ctx->h_sync, 64, cudaHostAllocDefault) != cudaSuccess) {
     ghb_ctx_destroy(ctx);
     return GHB_ERR_OOM;
   }
@@ -307,6 +326,7 @@ int32_t ghb_ctx_destroy(ghb_ctx* ctx) {
   if (ctx->lb_status) cudaFree(ctx->lb_status);
   if (ctx->gb_table) cudaFree(ctx->gb_table);
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
+  if (ctx->h_sync) cudaFreeHost(ctx->h_sync);
   for (int l = 0; l < kStageLanes; l++)
     for (int b = 0; b < 2; b++) {
       if (ctx->stage[l][b]) cudaFreeHost(ctx->stage[l][b]);
@@ -354,12 +374,18 @@ int32_t ghb_ctx_set_spin_limit(ghb_ctx* ctx, int32_t polls) {
   return GHB_OK;
 }
 
-int32_t ghb_sync(ghb_ctx* ctx, void* stream) {
+int32_t ghb_sync(ghb_ctx* ctx, void* stream) { return ghb_sync_count(ctx, nullptr, nullptr, stream); }
+
+int32_t ghb_sync_count(ghb_ctx* ctx, const int64_t* d_count, int64_t* count, void* stream) {
   if (!ctx) return GHB_ERR_INVALID;
   cudaStream_t s = (cudaStream_t)stream;
+  // the words come back in the stream's order, into pinned memory: one wait
+  GHB_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sync, ctx->d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  if (d_count)
+    GHB_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sync + 1, d_count, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   GHB_CUDA_TRY(ctx, cudaStreamSynchronize(s));
-  int32_t st = 0;
-  GHB_CUDA_TRY(ctx, cudaMemcpy(&st, ctx->d_status, sizeof(st), cudaMemcpyDeviceToHost));
+  if (d_count && count) *count = ctx->h_sync[1];
+  const int32_t st = *(const int32_t*)ctx->h_sync;
   if (st != 0) {
     GHB_CUDA_TRY(ctx, cudaMemset(ctx->d_status, 0, sizeof(st)));
     ctx->gb_dirty = true;  // a failed group-by may leave its table partly filled

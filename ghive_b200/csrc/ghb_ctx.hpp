@@ -46,6 +46,9 @@ struct ghb_ctx {
   // (ghb_ctx_set_spin_limit)
   int32_t spin_limit = ghb::kSpinLimit;
 
+  // pinned host words a sync reads back: the status word, a count
+  int64_t* h_sync = nullptr;
+
   // self-resetting counters: [0] tile claim, [1] finished CTAs, ...
   unsigned long long* d_counters = nullptr;
 
@@ -94,6 +97,9 @@ int32_t regrow(ghb_ctx* ctx, void** buf, size_t* bytes, size_t want, cudaStream_
 // opt-in maximum): changing a kernel's attributes on every call would put a
 // runtime call that may wait on running work into every launch path.
 int32_t ensure_dyn_smem(ghb_ctx* ctx, const void* fn, size_t bytes);
+// CTAs of `threads` threads and `smem` dynamic bytes of kernel `fn` that an SM
+// of the current device holds (at least 1); asked once per kernel and shape.
+int32_t resident_ctas(ghb_ctx* ctx, const void* fn, int threads, size_t smem, int* per_sm);
 }  // namespace ghb
 
 struct ghb_join_table {

@@ -418,7 +418,7 @@ int32_t filter_impl(ghb_ctx* ctx, const ghb_predicate* pred, const ghb_column* c
     return GHB_OK;
   }
   int per_sm = 0;
-  GHB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, filter_kernel, kFiltThreads, 0));
+  if ((st = resident_ctas(ctx, (const void*)filter_kernel, kFiltThreads, 0, &per_sm))) return st;
   const int64_t slots = (int64_t)ctx->num_sms * std::max(1, per_sm);
   // one range per resident CTA where the rows allow, in whole tiles
   const int64_t ntiles = (n + kFiltTile - 1) / kFiltTile;

@@ -511,8 +511,7 @@ int32_t filter_groupby_impl(ghb_ctx* ctx, const ghb_predicate* pred, const ghb_c
   const int threads = su.threads;
   int blocks_per_sm = 0;
   if (int32_t ast = ensure_dyn_smem(ctx, kfn, smem)) return ast;
-  GHB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, kfn, threads, smem));
-  blocks_per_sm = std::max(1, blocks_per_sm);
+  if (int32_t ost = resident_ctas(ctx, kfn, threads, smem, &blocks_per_sm)) return ost;
   if (cfg && cfg->ctas_per_sm > 0) blocks_per_sm = std::min(blocks_per_sm, cfg->ctas_per_sm);
   int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->num_sms * blocks_per_sm, p.ntiles));
   void* args[] = {&p};

@@ -82,7 +82,42 @@ struct Entry {
   bool failed = false;
 };
 
+// What fixes a kernel's source (jit_groupby_source), as bytes: the key by which
+// a call finds its kernel without writing the source.
+std::string signature(const GbParams& p, bool keyed, bool batch, int threads, int dev) {
+  std::string s;
+  auto put = [&](int v) { s.append((const char*)&v, sizeof(v)); };
+  auto col = [&](int c) {
+    put(c);
+    if (c >= 0) put(p.cols.c[c].type * 4 + p.cols.c[c].null_mode);
+  };
+  put(dev);
+  put(p.tile_rows);
+  put(threads);
+  put((keyed ? 1 : 0) + (batch ? 2 : 0) + (p.warp_agg ? 4 : 0));
+  col(keyed ? p.key_col : -1);
+  put(p.pred.n_nodes);
+  for (int k = 0; k < p.pred.n_nodes; k++) {
+    const ghb_pred_node& nd = p.pred.nodes[k];
+    put(nd.mode);
+    if (nd.mode == GHB_FILTER_AND || nd.mode == GHB_FILTER_OR) {
+      put(nd.child[0]);
+      put(nd.child[1]);
+    } else {
+      col(nd.col);
+      col(nd.col2);
+      put(nd.lit_is_double ? 1 : 0);
+    }
+  }
+  for (int a = 0; a < p.acc.n_acc; a++) {
+    put(p.acc.kind[a]);
+    col(p.acc.col[a]);
+  }
+  return s;
+}
+
 std::mutex g_mu;
+std::unordered_map<std::string, const void*> g_known;   // key: signature
 std::unordered_map<std::string, Entry> g_cache;   // key: device + source
 
 std::string cache_dir() {
@@ -184,11 +219,14 @@ const void* jit_groupby_kernel(const GbParams& p, bool keyed, bool batch, int th
   }
   if (threads <= 0 || p.tile_rows % threads || p.tile_rows / threads < 1 || p.tile_rows / threads > kGbRows)
     return nullptr;
+  const std::string sig = signature(p, keyed, batch, threads, dev);
+  std::lock_guard<std::mutex> g(g_mu);
+  auto known = g_known.find(sig);
+  if (known != g_known.end()) return known->second;
   const std::string src = jit_groupby_source(p, keyed, batch, threads);
   const std::string key = std::to_string(dev) + "\n" + src;
-  std::lock_guard<std::mutex> g(g_mu);
   auto it = g_cache.find(key);
-  if (it != g_cache.end()) return it->second.failed ? nullptr : (const void*)it->second.kern;
+  if (it != g_cache.end()) return g_known[sig] = it->second.failed ? nullptr : (const void*)it->second.kern;
   Entry e;
   // a cubin compiled earlier, by source, header and compiler version
   uint64_t h = fnv1a(src);
@@ -224,7 +262,7 @@ const void* jit_groupby_kernel(const GbParams& p, bool keyed, bool batch, int th
     e.failed = true;
   }
   g_cache[key] = e;
-  return e.failed ? nullptr : (const void*)e.kern;
+  return g_known[sig] = e.failed ? nullptr : (const void*)e.kern;
 }
 
 }  // namespace ghb

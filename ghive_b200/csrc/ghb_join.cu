@@ -1098,22 +1098,22 @@ int32_t join_probe_impl(ghb_ctx* ctx, const ghb_join_table* t, const ghb_column*
 #undef GHB_COUNT
   p.dup_bit = t->slots + 4 <= (1ll << 30) ? 1 << 30 : 0;
   int per_sm = 0;
-  GHB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, count_kernel, threads, 0));
+  if ((st = resident_ctas(ctx, (const void*)count_kernel, threads, 0, &per_sm))) return st;
   int grid = (int)std::min<int64_t>(p.nchunks, (int64_t)ctx->num_sms * std::max(1, per_sm));
   count_kernel<<<grid, threads, 0, stream>>>(p);
   GHB_LAUNCH_CHECK(ctx);
   // the count pass of a direct table (the build decided on the device which one works)
-  GHB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, count_direct, threads, 0));
+  if ((st = resident_ctas(ctx, (const void*)count_direct, threads, 0, &per_sm))) return st;
   grid = (int)std::min<int64_t>(p.nchunks, (int64_t)ctx->num_sms * std::max(1, per_sm));
   count_direct<<<grid, threads, 0, stream>>>(p);
   GHB_LAUNCH_CHECK(ctx);
   if ((st = scan_counts(ctx, p.chunk_count, nunits, d_out_rows, stream))) return st;
-  GHB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, write_kernel, threads, 0));
+  if ((st = resident_ctas(ctx, (const void*)write_kernel, threads, 0, &per_sm))) return st;
   grid = (int)std::min<int64_t>(p.nchunks, (int64_t)ctx->num_sms * std::max(1, per_sm));
   write_kernel<<<grid, threads, 0, stream>>>(p);
   GHB_LAUNCH_CHECK(ctx);
   if (p.lean && !p.out_brow) {   // the lean write pass, when the build's keys turn out unique
-    GHB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, write_lean, kJThreads, 0));
+    if ((st = resident_ctas(ctx, (const void*)write_lean, kJThreads, 0, &per_sm))) return st;
     grid = (int)std::min<int64_t>((nunits * 32 + kJThreads - 1) / kJThreads, (int64_t)ctx->num_sms * std::max(1, per_sm));
     write_lean<<<grid, kJThreads, 0, stream>>>(p);
   }

@@ -62,32 +62,28 @@ class _Cols:
 
     def __init__(self, cols):
         self.keep = []
-        descs = []
-        for c in cols:
+        self.n = len(cols)
+        self.arr = (abi.Column * max(1, self.n))()
+        for c, d in zip(cols, self.arr):
             v, isnull, mode = _split(c)
             if isinstance(v, tuple):   # ("string", utf-8 bytes, int32 [start,end) pairs)
                 _, chars, idx = v
-                d = abi.Column()
                 d.type, d.null_mode = abi.STRING, abi.NULLS_NONE
                 d.data, d.aux, d.n = _ptr(chars), _ptr(idx), len(idx) // 2
                 self.keep += [chars, idx]
-                descs.append(d)
                 continue
             if torch is not None and isinstance(v, torch.Tensor):
                 v = v.contiguous()
-                if isnull is not None:
-                    isnull = isnull.to(torch.uint8).contiguous()
+                if isnull is not None:   # a bool map is bytes of 0 and 1 already
+                    isnull = (isnull.view(torch.uint8) if isnull.dtype == torch.bool else
+                              isnull.to(torch.uint8)).contiguous()
             else:
                 v = np.ascontiguousarray(v)
                 if isnull is not None:
                     isnull = np.ascontiguousarray(isnull, dtype=np.uint8)
-            d = abi.Column()
             d.type, d.null_mode = _dtype_code(v), mode
             d.data, d.is_null, d.n = _ptr(v), _ptr(isnull), len(v)
             self.keep += [v, isnull]
-            descs.append(d)
-        self.n = len(descs)
-        self.arr = (abi.Column * max(1, self.n))(*descs)
 
     def __getitem__(self, i):
         return self.arr[i]
@@ -103,6 +99,8 @@ class _Outs:
     def __init__(self, types, cap, device=None, with_nulls=True):
         self.cols = []
         descs = []
+        if isinstance(device, str):
+            device = torch.device(device)
         for t in types:
             n = max(1, cap)
             if t == abi.STRING:   # [start,end) pairs into the input column's bytes
@@ -134,9 +132,14 @@ class _Outs:
     def rows(self, k):
         out = []
         for (d, nl), o in zip(self.cols, self.arr):
-            d = d[:2 * k] if o.type == abi.STRING else d[:k]
-            out.append((d, None if nl is None else nl[:k].bool() if torch is not None and
-                        isinstance(nl, torch.Tensor) else nl[:k].astype(bool)))
+            m = 2 * k if o.type == abi.STRING else k
+            if len(d) != m:
+                d = d[:m]
+            if nl is not None and len(nl) != k:
+                nl = nl[:k]
+            # the kernels write 0 or 1: a device map's bytes are a bool tensor's
+            out.append((d, None if nl is None else nl.view(torch.bool) if torch is not None and
+                        isinstance(nl, torch.Tensor) else nl.astype(bool)))
         return out
 
 
@@ -147,11 +150,15 @@ def _pred(pred):
     return C.addressof(s), s
 
 
+_has_cuda = None
+
+
 def _stream(stream):
+    global _has_cuda
     if stream is None:
-        if torch is not None and torch.cuda.is_available():
-            return torch.cuda.current_stream().cuda_stream
-        return None
+        if _has_cuda is None:
+            _has_cuda = torch is not None and torch.cuda.is_available()
+        return torch.cuda.current_stream().cuda_stream if _has_cuda else None
     return stream if isinstance(stream, int) else stream.cuda_stream
 
 
@@ -249,6 +256,12 @@ class Context:
     def sync(self, stream=None):
         self._check(lib().ghb_sync(self.h, _stream(stream)))
 
+    def _sync_count(self, d_count, stream):
+        """sync() and the device count a call wrote, in one wait."""
+        n = C.c_int64()
+        self._check(lib().ghb_sync_count(self.h, d_count.data_ptr(), C.byref(n), stream))
+        return n.value
+
     def set_spin_limit(self, polls):
         """Bound of this context's look-back waits (polls <= 0: the default)."""
         self._check(lib().ghb_ctx_set_spin_limit(self.h, int(polls)))
@@ -275,14 +288,14 @@ class Context:
         if outs is None:
             outs = _Outs([cs[j].type for j in proj], cap, self.torch_device, with_nulls=with_nulls)
         pa = (C.c_int32 * max(1, len(proj)))(*proj)
-        d_rows = torch.zeros(1, dtype=torch.int64, device=self.torch_device)
+        d_rows = torch.empty(1, dtype=torch.int64, device=self.torch_device)  # the kernel writes it
         pp, keep = _pred(pred)
+        stream = _stream(stream)
         self._check(lib().ghb_filter(self.h, pp, cs.ptr, cs.n, pa, len(proj), outs.ptr, cap,
-                                     d_rows.data_ptr(), _stream(stream)))
+                                     d_rows.data_ptr(), stream))
         if not sync:
             return outs, d_rows
-        self.sync(stream)
-        k = int(d_rows.item())
+        k = self._sync_count(d_rows, stream)
         return outs.rows(min(k, cap)), k
 
     def filter_groupby(self, pred, cols, keys, aggs, capacity=None, max_groups=None, cfg=None,
@@ -304,13 +317,13 @@ class Context:
             cfg.max_groups = max_groups
         d_groups = torch.empty(1, dtype=torch.int64, device=self.torch_device)  # the finalize writes it
         pp, keep = _pred(pred)
+        stream = _stream(stream)
         self._check(lib().ghb_filter_groupby(self.h, pp, cs.ptr, cs.n, ka, len(keys), ag, len(aggs),
                                              outs.ptr, cap, d_groups.data_ptr(), C.byref(cfg),
-                                             _stream(stream)))
+                                             stream))
         if not sync:
             return outs, d_groups
-        self.sync(stream)
-        g = int(d_groups.item())
+        g = self._sync_count(d_groups, stream)
         res = outs.rows(min(g, cap))
         return res[:len(keys)], res[len(keys):], g
 
@@ -378,16 +391,16 @@ class Context:
             op = _Outs([ppl[j].type for j in range(ppl.n)], capacity, self.torch_device)
             prow = torch.empty(capacity, dtype=torch.int32, device=self.torch_device) if rowids else None
             brow = torch.empty(capacity, dtype=torch.int32, device=self.torch_device) if rowids else None
-            d_rows = torch.zeros(1, dtype=torch.int64, device=self.torch_device)
+            d_rows = torch.empty(1, dtype=torch.int64, device=self.torch_device)  # the probe writes it
             outs = (ob, op, prow, brow, d_rows)
         ob, op, prow, brow, d_rows = outs
+        stream = _stream(stream)
         self._check(lib().ghb_join_probe(self.h, table.handle, pk.ptr, join_type, ob.ptr,
                                          ppl.ptr, ppl.n, op.ptr, _ptr(prow), _ptr(brow),
-                                         capacity, d_rows.data_ptr(), _stream(stream)))
+                                         capacity, d_rows.data_ptr(), stream))
         if not sync:
             return outs
-        self.sync(stream)
-        k = int(d_rows.item())
+        k = self._sync_count(d_rows, stream)
         m = min(k, capacity)
         return {"rows": k, "probe_rowid": None if prow is None else prow[:m],
                 "build_rowid": None if brow is None else brow[:m],

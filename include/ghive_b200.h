@@ -213,6 +213,9 @@ int32_t ghb_abi_version(void);
 /* Waits for `stream` and returns the first device-side error recorded on the
  * context since the previous ghb_sync (GHB_OK if none), then clears it. */
 int32_t ghb_sync(ghb_ctx* ctx, void* stream);
+/* The same, and with it, in one wait, the device int64 *d_count that a call
+ * before it on `stream` wrote (a row or group count), to *count. */
+int32_t ghb_sync_count(ghb_ctx* ctx, const int64_t* d_count, int64_t* count, void* stream);
 /* Number of kernels the context launched since creation. */
 int64_t ghb_kernel_launches(const ghb_ctx* ctx);
 /* Bound of the decoupled look-back waits (filter, join probe offsets, sort
