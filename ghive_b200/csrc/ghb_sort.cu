@@ -1293,7 +1293,13 @@ __global__ void __launch_bounds__(kLongThreads) sort_finish_long_kernel(const __
   }
 }
 
-// Output in input order (keys all equal, or n tiny): gathers row r to r, or
+}  // namespace ghb
+
+#include "ghb_sort_small.cuh"
+
+namespace ghb {
+
+// Output in input order (keys all equal): gathers row r to r, or
 // row perm[r] to r when a permutation is given.
 template <typename V>
 __global__ void sort_identity_kernel(PassParams p, const V* perm) {
@@ -1381,8 +1387,8 @@ static int32_t run_passes(ghb_ctx* ctx, PassParams& pp, const std::vector<Segmen
   const size_t dyn = (size_t)kSortTile * 8;
   if ((st = set_smem<V>(ctx, dyn))) return st;
   int per_sm = 0;
-  GHB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                        &per_sm, sort_pass_kernel<V, kSrcPacked, kDstPacked>, kSortThreads, dyn));
+  if ((st = resident_ctas(ctx, (const void*)sort_pass_kernel<V, kSrcPacked, kDstPacked>, kSortThreads, dyn, &per_sm)))
+    return st;
   int pgrid = (int)std::min<int64_t>(pp.ntiles, (int64_t)ctx->num_sms * std::max(1, per_sm));
   int done = 0;
   bool have_perm = false;  // a previous pass left the row order in vb[cur]
@@ -1486,6 +1492,8 @@ int32_t sort_impl(ghb_ctx* ctx, const ghb_column* keys, const int32_t* orders,
     int no = null_orders ? null_orders[j] : GHB_NULLS_DEFAULT;
     K.k[j].nulls_first = no == GHB_NULLS_FIRST || (no == GHB_NULLS_DEFAULT && !K.k[j].desc);
   }
+  if (n <= kSmallRows)
+    return sort_small(ctx, K, payload, npayload, out_keys, out_payload, out_rowid, n, stream);
   // one zeroed block: the analysis, the histograms, the count of long runs
   unsigned long long* d_mm = nullptr;
   const size_t stat_bytes = align256(kStatWords * 8), hist_bytes = (size_t)kMaxSeg * kMaxPasses * kBins * 4;
