@@ -50,7 +50,6 @@ __global__ void __launch_bounds__(kGbThreads) gb_batch_fold_kernel(BatchParams b
 }
 
 __global__ void __launch_bounds__(kFinThreads) gb_batch_finalize_kernel(BatchFinParams b) {
-  __shared__ uint64_t rb[kFinThreads * (kMaxAcc + 1)];
   const int64_t total = b.choff[b.ninst];
   for (int64_t ch = blockIdx.x; ch < total; ch += gridDim.x) {
     // the instance of unit ch: the last i with choff[i] <= ch
@@ -62,8 +61,8 @@ __global__ void __launch_bounds__(kFinThreads) gb_batch_finalize_kernel(BatchFin
     }
     const FinParams& f = b.fins[lo];
     const int64_t local = ch - b.choff[lo];
-    finalize_unit(f, local, rb);
-    if (local == 0 && threadIdx.x == 0) finalize_sides(f, rb);
+    finalize_unit(f, local);
+    if (local == 0 && threadIdx.x == 0) finalize_sides(f);
   }
   __shared__ int last;
   __syncthreads();

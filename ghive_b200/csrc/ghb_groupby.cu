@@ -37,11 +37,10 @@ __global__ void __launch_bounds__(kGbThreads) gb_fold_kernel(GbParams p) {
   fold_kernel_body<GenericFolder<KEYED, NULLABLE>>(p);
 }
 
-__global__ void __launch_bounds__(kFinThreads) gb_finalize_kernel(FinParams f) {
-  __shared__ uint64_t rb[kFinThreads * (kMaxAcc + 1)];
+__global__ void __launch_bounds__(kFinThreads, 4) gb_finalize_kernel(const __grid_constant__ FinParams f) {
   const int64_t nu = fin_units(f.C);
-  for (int64_t u = blockIdx.x; u < nu; u += gridDim.x) finalize_unit(f, u, rb);
-  if (blockIdx.x == 0 && threadIdx.x == 0) finalize_sides(f, rb);
+  for (int64_t u = blockIdx.x; u < nu; u += gridDim.x) finalize_unit(f, u);
+  if (blockIdx.x == 0 && threadIdx.x == 0) finalize_sides(f);
   // the last CTA to finish publishes the group count and resets the counters
   __syncthreads();
   if (threadIdx.x == 0) {
