@@ -26,6 +26,7 @@
 #include <algorithm>
 
 #include "ghb_ctx.hpp"
+#include "ghb_range.cuh"
 
 namespace ghb {
 
@@ -37,63 +38,59 @@ struct KpMinMaxParams {
   int32_t nkeys;
   ghb_column col[kMaxPackKeys];
   int64_t n;
-  unsigned long long* out;   // per key: [0] min image, [1] max image, [2] any NULL
+  unsigned long long* out;   // per key: [0] max of ~image (~min), [1] max image, [2] any NULL; zeroed
 };
 
-__global__ void __launch_bounds__(256) keypack_minmax_kernel(KpMinMaxParams p) {
-  __shared__ unsigned long long s_red[3][8];
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int warp = threadIdx.x >> 5;
-  for (int j = 0; j < p.nkeys; j++) {
-    const ghb_column c = p.col[j];
-    unsigned long long mn = ~0ull, mx = 0, anynull = 0;
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < p.n; r += stride) {
-      const int64_t raw = ld_raw_cs(c, r);
-      if (c.null_mode != GHB_NULLS_NONE && raw_is_null(c, raw, r)) {
-        anynull = 1;
-        continue;
-      }
-      const unsigned long long img = kp_image(c, raw);
-      mn = min(mn, img);
-      mx = max(mx, img);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      mn = min(mn, __shfl_down_sync(0xffffffffu, mn, o));
-      mx = max(mx, __shfl_down_sync(0xffffffffu, mx, o));
-      anynull |= __shfl_down_sync(0xffffffffu, anynull, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      s_red[0][warp] = mn;
-      s_red[1][warp] = mx;
-      s_red[2][warp] = anynull;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {   // one set of atomics per CTA
-      for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
-        mn = min(mn, s_red[0][w]);
-        mx = max(mx, s_red[1][w]);
-        anynull |= s_red[2][w];
-      }
-      atomicMin(&p.out[3 * j], mn);
-      atomicMax(&p.out[3 * j + 1], mx);
-      if (anynull) atomicOr(&p.out[3 * j + 2], 1ull);
-    }
-    __syncthreads();
-  }
+__global__ void __launch_bounds__(256) keypack_minmax_kernel(const __grid_constant__ KpMinMaxParams p) {
+  for (int j = 0; j < p.nkeys; j++) range_to(p.col[j], p.n, false, p.out + 3 * j);
 }
 
-__global__ void __launch_bounds__(256) keypack_pack_kernel(KeyPackPlan p, int64_t n, int64_t* out) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
-       r += (int64_t)gridDim.x * blockDim.x) {
+// A row's field of key j (NULL: nothing), in its place.
+__device__ __forceinline__ uint64_t kp_field(const KeyPackPlan& p, int j, int64_t raw, bool null) {
+  uint64_t v = 0;
+  if (p.fshift[j] >= 0 && !null) v |= 1ull << p.fshift[j];
+  if (!null && p.vbits[j] > 0) v |= (kp_image(p.col[j], raw) - p.umin[j]) << p.vshift[j];
+  return v;
+}
+
+// Packs the keys.  With `vec` (16-byte aligned columns and output, NULL maps
+// aligned to 4) four rows a thread by 16-byte loads and stores; the rows past
+// them, or all, one at a time.  Two INT keys, one with a NULL map, of 12M rows:
+// 79 us a row at a time (loads in a chain), 57 us now; their ranges 121 ->
+// 24 us.
+__global__ void __launch_bounds__(256) keypack_pack_kernel(const __grid_constant__ KeyPackPlan p, int64_t n,
+                                                           int64_t* out, int vec) {
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int64_t done = 0;
+  if (vec) {
+    for (int64_t g = tid; g < n / 4; g += stride) {
+      uint64_t v[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int j = 0; j < kMaxPackKeys; j++) {
+        if (j >= p.nkeys) break;
+        const ghb_column& c = p.col[j];
+        int64_t raw[4];
+        load4(c, g * 4, raw);
+        const bool map = c.null_mode == GHB_NULLS_BYTEMAP;
+        const unsigned int b = map ? __ldcs((const unsigned int*)c.is_null + g) : 0;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+          v[u] |= kp_field(p, j, raw[u], map ? (b >> (8 * u) & 0xffu) != 0 : raw_is_null(c, raw[u], 0));
+      }
+      ulonglong2* o = (ulonglong2*)out + g * 2;
+      __stcs(o, make_ulonglong2(v[0], v[1]));
+      __stcs(o + 1, make_ulonglong2(v[2], v[3]));
+    }
+    done = n / 4 * 4;
+  }
+  for (int64_t r = done + tid; r < n; r += stride) {
     uint64_t v = 0;
 #pragma unroll
     for (int j = 0; j < kMaxPackKeys; j++) {
       if (j >= p.nkeys) break;
-      const ghb_column& c = p.col[j];
-      const int64_t raw = ld_raw_cs(c, r);
-      const bool null = c.null_mode != GHB_NULLS_NONE && raw_is_null(c, raw, r);
-      if (p.fshift[j] >= 0 && !null) v |= 1ull << p.fshift[j];
-      if (!null && p.vbits[j] > 0) v |= (kp_image(c, raw) - p.umin[j]) << p.vshift[j];
+      const int64_t raw = ld_raw_cs(p.col[j], r);
+      v |= kp_field(p, j, raw, raw_is_null(p.col[j], raw, r));
     }
     __stcs((unsigned long long*)out + r, (unsigned long long)v);
   }
@@ -244,13 +241,7 @@ int32_t keypack_prepare(ghb_ctx* ctx, const ghb_column* cols, const int32_t* key
   unsigned long long* d_mm = nullptr;
   int32_t st = scratch_alloc(ctx, 3 * 8 * kMaxPackKeys, (void**)&d_mm, stream);
   if (st) return st;
-  unsigned long long init[3 * kMaxPackKeys];
-  for (int j = 0; j < kMaxPackKeys; j++) {
-    init[3 * j] = ~0ull;
-    init[3 * j + 1] = 0;
-    init[3 * j + 2] = 0;
-  }
-  GHB_CUDA_TRY(ctx, cudaMemcpyAsync(d_mm, init, sizeof(init), cudaMemcpyHostToDevice, stream));
+  GHB_CUDA_TRY(ctx, cudaMemsetAsync(d_mm, 0, 3 * 8 * kMaxPackKeys, stream));
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)ctx->num_sms * 8));
   mp.out = d_mm;
   keypack_minmax_kernel<<<grid, 256, 0, stream>>>(mp);
@@ -260,9 +251,8 @@ int32_t keypack_prepare(ghb_ctx* ctx, const ghb_column* cols, const int32_t* key
   GHB_CUDA_TRY(ctx, cudaStreamSynchronize(stream));
   int bits = 0;
   for (int j = 0; j < nkeys; j++) {
-    const bool anyval = mm[3 * j] <= mm[3 * j + 1];
-    P.umin[j] = anyval ? mm[3 * j] : 0;
-    const uint64_t range = anyval ? mm[3 * j + 1] - mm[3 * j] : 0;
+    uint64_t range;
+    key_range(mm + 3 * j, &P.umin[j], &range);
     P.vbits[j] = (int8_t)(range == 0 ? 0 : 64 - __builtin_clzll(range));
     P.vshift[j] = (int8_t)bits;
     bits += P.vbits[j];
@@ -277,7 +267,11 @@ int32_t keypack_prepare(ghb_ctx* ctx, const ghb_column* cols, const int32_t* key
     }
   }
   *too_wide = false;
-  keypack_pack_kernel<<<grid, 256, 0, stream>>>(P, n, packed);
+  int vec = ((uintptr_t)packed & 15) == 0;
+  for (int j = 0; j < nkeys; j++)
+    vec &= ((uintptr_t)P.col[j].data & 15) == 0 &&
+           (P.col[j].null_mode != GHB_NULLS_BYTEMAP || ((uintptr_t)P.col[j].is_null & 3) == 0);
+  keypack_pack_kernel<<<grid, 256, 0, stream>>>(P, n, packed, vec);
   GHB_LAUNCH_CHECK(ctx);
   return GHB_OK;
 }
@@ -449,13 +443,7 @@ int32_t keypack_join(ghb_ctx* ctx, const ghb_column* a, const ghb_column* b, int
   unsigned long long* d_mm = nullptr;
   int32_t st = scratch_alloc(ctx, 3 * 8 * kMaxPackKeys, (void**)&d_mm, stream);
   if (st) return st;
-  unsigned long long init[3 * kMaxPackKeys];
-  for (int j = 0; j < kMaxPackKeys; j++) {
-    init[3 * j] = ~0ull;
-    init[3 * j + 1] = 0;
-    init[3 * j + 2] = 0;
-  }
-  GHB_CUDA_TRY(ctx, cudaMemcpyAsync(d_mm, init, sizeof(init), cudaMemcpyHostToDevice, stream));
+  GHB_CUDA_TRY(ctx, cudaMemsetAsync(d_mm, 0, 3 * 8 * kMaxPackKeys, stream));
   for (int side = 0; side < 2; side++) {
     const ghb_column* c = side ? b : a;
     KpMinMaxParams mp;
@@ -476,9 +464,8 @@ int32_t keypack_join(ghb_ctx* ctx, const ghb_column* a, const ghb_column* b, int
   P.nkeys = nkeys;
   int bits = 0;
   for (int j = 0; j < nkeys; j++) {
-    const bool anyval = mm[3 * j] <= mm[3 * j + 1];
-    P.umin[j] = anyval ? mm[3 * j] : 0;
-    const uint64_t range = anyval ? mm[3 * j + 1] - mm[3 * j] : 0;
+    uint64_t range;
+    key_range(mm + 3 * j, &P.umin[j], &range);
     P.vbits[j] = (int8_t)(range == 0 ? 0 : 64 - __builtin_clzll(range));
     P.vshift[j] = (int8_t)bits;
     P.fshift[j] = -1;
