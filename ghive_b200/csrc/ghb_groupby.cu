@@ -200,7 +200,9 @@ int32_t gb_setup(ghb_ctx* ctx, const ghb_predicate* pred, const ghb_column* cols
   int64_t max_groups = su.max_groups > 0 ? su.max_groups : out_capacity;
   if (nkeys == 0) max_groups = 1;
   max_groups = std::min<int64_t>(max_groups, std::max<int64_t>(n, 1));
-  const double lf = su.load_factor > 0.f ? std::min<double>(su.load_factor, 0.9) : 0.5;
+  const double lf = su.load_factor > 0.f ? std::min<double>(su.load_factor, 0.9)
+                    : su.roomy           ? gb_load_factor(max_groups, 1 + p.acc.n_acc)
+                                         : 0.5;
   int64_t C = next_pow2_i64(std::max<int64_t>((int64_t)((double)max_groups / lf) + 1, 64));
   if (C > (1ll << 30))
     return set_error(ctx, GHB_ERR_CAPACITY, "group-by table of %lld slots exceeds 2^30", (long long)C);
@@ -288,11 +290,7 @@ int32_t gb_setup(ghb_ctx* ctx, const ghb_predicate* pred, const ghb_column* cols
   p.stage_bytes = (off + 127) & ~127;
   p.tx_bytes = off;
   p.bulk = aligned ? 1 : 0;
-  // words per global record: the key and the accumulators; a table too big
-  // for L2 pads them to 2, 4, 8, 16 or 24 words so that the atomics of one
-  // row touch one aligned 16/32/64-byte block of a DRAM line
-  p.R = 1 + p.acc.n_acc;
-  if (C > (1ll << 17)) p.R = p.R <= 2 ? 2 : p.R <= 4 ? 4 : p.R <= 8 ? 8 : p.R <= 16 ? 16 : 24;
+  p.R = gb_record_words(1 + p.acc.n_acc, C);
   p.C = C;
   p.gshift = 64 - log2_exact(C);
   p.gprobe = (int32_t)std::min<int64_t>(C, 1 << 20);
@@ -453,6 +451,9 @@ int32_t filter_groupby_impl(ghb_ctx* ctx, const ghb_predicate* pred, const ghb_c
   su.warp_agg = -1;
   su.tile_rows = cfg ? cfg->tile_rows : 0;
   su.nstages = cfg ? cfg->nstages : 0;
+  // the allocation-free table's size is part of its contract, and a server
+  // slot's working memory was admitted by its size
+  su.roomy = fixed_table || ctx->stream_ordered ? 0 : 1;
   if (cfg && cfg->global_slots_log2 > 0) {
     // an explicit table size: the load factor that yields it
     if (cfg->global_slots_log2 > 30)

@@ -116,6 +116,27 @@ inline size_t gb_table_bytes(int64_t C, int32_t R) {
   return (size_t)(C + 2) * R * 8 + 16 + (size_t)(C / 32) * 4;
 }
 
+int64_t next_pow2_i64(int64_t v);
+
+// Words of a record of n words in a table of C hashed slots: a table too big
+// for L2 pads them to 2, 4, 8, 16 or 24 so that the atomics of one row touch
+// one aligned 16/32/64-byte block of a DRAM line.
+inline int32_t gb_record_words(int32_t n, int64_t C) {
+  return C <= (1ll << 17) ? n : n <= 2 ? 2 : n <= 4 ? 4 : n <= 8 ? 8 : n <= 16 ? 16 : 24;
+}
+
+// Load factor of a global table for `groups` groups of n record words.  Where
+// many rows go past the shared tables, a row walks the table with a dependent
+// load per probe, and shorter chains pay while the table is not much larger
+// than L2.  16M rows of the fact aggregates, fold at a load factor of 0.5 /
+// 0.25: 7000 groups 730 / 582 us, 20,000 628 / 597, 100,000 783 / 740, 1M (268
+// MB at 0.25) 885 / 833; at 537 MB 1848.  Up to 2048 groups the rows stay in
+// the shared tables, and the finalize would only visit more slots.
+inline double gb_load_factor(int64_t groups, int32_t n) {
+  const int64_t C = next_pow2_i64(4 * groups + 1);
+  return groups > 2048 && C * gb_record_words(n, C) * 8 <= (272ll << 20) ? 0.25 : 0.5;
+}
+
 // Points p/f at a zeroed table of gb_table_bytes(C, R) bytes at `base`.
 inline void gb_table_bind(void* base, int64_t C, int32_t R, GbParams* p, FinParams* f) {
   uint64_t* rec = (uint64_t*)base;
@@ -962,6 +983,7 @@ struct GbSetup {
   int64_t max_groups;   // table sizing: groups expected (0 = out_capacity)
   int32_t smem_slots;   // -1 none, 0 auto, else power of two
   float load_factor;    // hashed slots = next_pow2(groups / load_factor); 0 = 0.5
+  int32_t roomy;        // 1: with load_factor 0, a quarter where gb_load_factor finds it worth it
   int32_t threads;      // CTA size of the fold (512 or 1024)
   int32_t tile_rows;    // 0 = as large as shared memory allows (threads times 1, 2 or 4)
   int32_t smem_table_slots; // shared-memory slots the layout reserves (0 = smem_slots)
