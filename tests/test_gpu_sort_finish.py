@@ -88,3 +88,22 @@ def test_sorted_and_reversed_input(ctx):
     k = np.arange(n, dtype=np.int64) * 1_000_003
     check(ctx, [k], payload=[np.arange(n, dtype=np.int32)])
     check(ctx, [k[::-1].copy()], payload=[np.arange(n, dtype=np.int32)])
+
+
+@pytest.mark.parametrize("ties", ["none", "below", "equal"])
+@pytest.mark.parametrize("orders", [[abi.ASC, abi.ASC], [abi.DESC, abi.ASC]])
+def test_keys_wider_than_a_word(ctx, ties, orders):
+    """Keys of 69 and 128 bits: sorted by the leading 64 when those tell the
+    rows apart, by every bit when rows differ only below them or are equal."""
+    g = np.random.default_rng(11)
+    n = 300_007
+    i = g.integers(0, 24, n, dtype=np.int32)
+    j = g.integers(np.iinfo(np.int64).min, np.iinfo(np.int64).max, n, dtype=np.int64)
+    if ties != "none":
+        a, b = g.choice(n, (2, 400), replace=False)
+        i[b], j[b] = i[a], j[a] ^ (1 if ties == "below" else 0)
+    pay = [np.arange(n, dtype=np.int32), g.random(n)]
+    check(ctx, [i, j], orders, payload=pay)
+    check(ctx, [j, g.integers(np.iinfo(np.int64).min, np.iinfo(np.int64).max, n, dtype=np.int64)], orders,
+          payload=pay[:1])
+    check(ctx, [j, i], orders, payload=pay, nulls=[g.random(n) < 0.001, g.random(n) < 0.1])
