@@ -657,9 +657,12 @@ def bench_sort(ctx, args, dev, stream, peak, peak_kind):
         l0 = ctx.launches
         ctx.sort([dd, dk], payload=[dr], sync=False, outs=souts)
         ctx.sync()
-        # the sort launches a min/max and a histogram kernel, then one kernel
-        # per executed radix pass
-        passes = ctx.launches - l0 - 2
+        # the sort launches a min/max, a sample and a histogram kernel, then one
+        # kernel per executed radix pass; when it sorts by the leading digits
+        # alone, two finish kernels follow.  All 52 bits are seven passes.
+        kernels = ctx.launches - l0 - 3
+        finish = kernels < 7
+        passes = kernels - 2 if finish else kernels
         times = []
         for _ in range(max(3, min(args.steps, 10))):
             a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -669,7 +672,7 @@ def bench_sort(ctx, args, dev, stream, peak, peak_kind):
             times.append((a, b))
         ctx.sync()
         ms = statistics.median(x.elapsed_time(y) for x, y in times)
-        per_pass_bytes = N_SORT * 12 + passes * N_SORT * 24 + N_SORT * 16
+        per_pass_bytes = N_SORT * (12 + 28 + passes * 24 + (28 if finish else 4))
         # e2e: pinned host columns through ghb_sort_host
         hd, hk, hr = pinned(d), pinned(k), pinned(rowid)
         hok = pinned_outs([abi.INT, abi.LONG], N_SORT, with_nulls=False)
@@ -685,9 +688,10 @@ def bench_sort(ctx, args, dev, stream, peak, peak_kind):
                                              "(read d 4 + k 8 + rowid 4, write 16)"),
                  "roofline_per_pass_formula": roofline(
                      per_pass_bytes, ms, peak, peak_kind,
-                     kernel="whole sort against N*12 + P*N*24 + N*16 bytes, P = %d executed "
-                            "radix passes" % passes,
-                     traffic=profile_traffic("sort_passes_20M.md")),
+                     kernel="whole sort against its kernels' bytes per row: ranges 12, packing 28, "
+                            "24 for each of %d radix passes%s" % (
+                                passes, ", finish 28" if finish else ", 4 more for decoding"),
+                     traffic=None if zipf else profile_traffic("sort_passes_20M.md")),
                  "e2e": {"value": N_SORT / (e2e_ms / 1e3), "unit": "rows/s", "ms_per_step": e2e_ms,
                          "h2d_bytes_per_step": N_SORT * 16, "d2h_bytes_per_step": N_SORT * 16,
                          "api": "ghb_sort_host (pinned host columns)"}}
