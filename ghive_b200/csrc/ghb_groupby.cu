@@ -222,7 +222,7 @@ int32_t gb_setup(ghb_ctx* ctx, const ghb_predicate* pred, const ghb_column* cols
   size_t row_bytes = 0;
   for (int c = 0; c < ncols; c++)
     if (used[c]) row_bytes += type_width(cols[c].type) + (cols[c].null_mode == GHB_NULLS_BYTEMAP ? 1 : 0);
-  const size_t smem_cap = 225 * 1024 - (size_t)std::max(0, su.extra_smem);
+  size_t smem_cap = 225 * 1024 - (size_t)std::max(0, su.extra_smem);
   int slot_words = 2 * (1 + p.acc.n_acc);
   if (su.narrow) {
     slot_words = (nkeys && cols[key_cols[0]].type == GHB_INT) ? 1 : 2;
@@ -243,6 +243,28 @@ int32_t gb_setup(ghb_ctx* ctx, const ghb_predicate* pred, const ghb_column* cols
     return set_error(ctx, GHB_ERR_INVALID, "nstages %d outside [2,%d]", su.nstages, kGbMaxStages);
   if (su.smem_slots == 0)
     while (S > 64 && table_bytes_smem(S) + 2 * stage_bytes_of(threads) > smem_cap) S /= 2;
+  // Rows that go past the shared table wait for the global one, and their loads
+  // and atomics in flight are held by the L1 that shared memory leaves over (28
+  // KB at 225 KB, 60 KB at 195, 92 at 163).  With many groups the CTA keeps
+  // within 195 KB, where a table halved for it (not below 1024 slots) and the
+  // tile it would have anyway fit.  Fold of 16M rows of the fact aggregates at
+  // 225 / 195 KB, 90 % of them passing: LONG keys (2048 / 1024 slots) 100,000
+  // groups 758 / 670 us, 1M 821 / 714, 50,000 685 / 690 (30 % passing: 339 /
+  // 326); INT keys (4096 / 2048) 50,000 636 / 617, 1M 836 / 679.  163 KB leaves
+  // a row per thread: 1M groups 682, but with 30 % passing 391 where 225 KB
+  // takes 387.  Below 32,768 groups the larger table keeps more rows: INT keys,
+  // 20,000 groups 516 / 590.
+  if (nkeys && su.tile_rows == 0 && su.nstages == 0 && S > 0 && max_groups > 32768) {
+    const size_t cap = std::min<size_t>(smem_cap, 195 * 1024);
+    int s = S, t = kGbRows * threads;
+    while (t > threads && table_bytes_smem(S) + 2 * stage_bytes_of(t) > smem_cap) t /= 2;
+    if (su.smem_slots == 0)
+      while (s > 1024 && table_bytes_smem(s) + 2 * stage_bytes_of(t) > cap) s /= 2;
+    if (table_bytes_smem(s) + 2 * stage_bytes_of(t) <= cap) {
+      S = s;
+      smem_cap = cap;
+    }
+  }
   reserve = std::max(S, su.smem_table_slots);
   if (table_bytes_smem(reserve) + 2 * stage_bytes_of(threads) > smem_cap)
     return set_error(ctx, GHB_ERR_UNSUPPORTED,

@@ -65,6 +65,20 @@ def test_every_aggregate_around_the_unit_change(ctx, groups):
     check(ctx, [key, q], [g.random(n) < 0.1, None], [0], [(abi.SUM, 1)], groups + 1)   # a NULL group; an odd record
 
 
+# Around the number of groups from which the fold leaves more of an SM to its
+# L1 and halves its shared table for that (LONG keys 2048 slots, INT 4096).
+@pytest.mark.parametrize("dtype", [np.int32, np.int64])
+@pytest.mark.parametrize("groups", [4096, 4097, 8192, 8193, 16_385, 32_768, 32_769])
+def test_shared_memory_left_to_the_cache(ctx, groups, dtype):
+    rng = np.random.default_rng(groups)
+    n = 3 * groups + 17
+    k = rng.permutation(np.arange(n) % groups).astype(dtype) - 5
+    qty, price, d = (rng.integers(1, 51, n), rng.integers(100, 10_000, n) / 100.0,
+                     rng.integers(0, 2526, n, dtype=np.int32))
+    aggs = [(abi.CNT, -1), (abi.SUM, 1), (abi.SUM, 2), (abi.AVG, 2), (abi.MIN, 3), (abi.MAX, 3)]
+    check(ctx, [k, qty, price, d], [None] * 4, [0], aggs, groups)
+
+
 @pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 70_001])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_packed_keys_off_the_vector_path(ctx, n, shift):
