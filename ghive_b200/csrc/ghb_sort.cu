@@ -856,8 +856,8 @@ __device__ __noinline__ int row_order(const PassParams& p, int64_t a, int64_t b)
 }
 
 // One run of len <= N rows from row a on, put in order by one thread: words
-// (field, place in the run) sorted in registers, then the rows that differ
-// only below the field by insertion.
+// (field, place in the run) sorted in registers, then, when equal words may be
+// of different keys (`partial`), those rows by insertion.
 template <int N, typename BELOW>
 __device__ __forceinline__ void sort_run(const uint32_t* s_word, uint16_t* s_src, int a, int len, bool partial,
                                          const BELOW& below) {
@@ -914,7 +914,10 @@ __global__ void __launch_bounds__(kSortThreads) sort_finish_kernel(const __grid_
   const unsigned long long* keys_in = (const unsigned long long*)p.keys_in + t0;
   const V* vals_in = (const V*)p.vals_in + t0;
   const uint64_t lead = ~0ull << p.shift;                // 0 < p.shift < 64
-  const int fshift = max(0, p.shift - kFinField);   // above 0 for a wide key, whose shift is 32 at least
+  const int fshift = max(0, p.shift - kFinField);
+  // equal words may be of keys that differ: below the field, or of a wide key
+  // below its leading 64 bits, however few of those the passes left
+  const bool partial = WIDE || fshift > 0;
   // row i's key is below row j's (of a wide key: by the bits left out, too)
   auto below = [&](int i, int j) -> bool {
     const uint64_t x = s_key[i], y = s_key[j];
@@ -1040,13 +1043,13 @@ __global__ void __launch_bounds__(kSortThreads) sort_finish_kernel(const __grid_
   }
   for (int r = threadIdx.x; r < n16; r += kSortThreads) {
     const int e = s_run[kRuns - 1 - r];
-    sort_run<16>(s_word, s_src, e & 2047, (e >> 11) + 1, fshift > 0, below);
+    sort_run<16>(s_word, s_src, e & 2047, (e >> 11) + 1, partial, below);
   }
   // the other way round, so that the warps without a run above go first
   for (int r = kSortThreads - 1 - threadIdx.x; r < n8; r += kSortThreads) {
     const int e = s_run[r], a = e & 2047, len = (e >> 11) + 1;
-    if (__any_sync(__activemask(), len > 4)) sort_run<8>(s_word, s_src, a, len, fshift > 0, below);
-    else sort_run<4>(s_word, s_src, a, len, fshift > 0, below);
+    if (__any_sync(__activemask(), len > 4)) sort_run<8>(s_word, s_src, a, len, partial, below);
+    else sort_run<4>(s_word, s_src, a, len, partial, below);
   }
   __syncthreads();
   for (int h = 0; h < kFinTile && h < end; h += kSortThreads * kFinItems) {
