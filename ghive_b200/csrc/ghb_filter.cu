@@ -134,7 +134,7 @@ __device__ __forceinline__ uint32_t leaf_bits(const FilterParams& p, int node, i
 
 // Writes column c's values of kFiltItems listed rows (rows[k] from `base` on,
 // k with bit k of `live`) to output rows out0 + i0 + k * kFiltThreads: every
-// load is issued before the stores.
+// load is issued before the stores.  A STRING's NULL map is string_nulls'.
 template <typename T>
 __device__ __forceinline__ void copy_rows(const ghb_column& c, const T* src, const ghb_out_column& o, int64_t base,
                                           const uint32_t (&rows)[kFiltItems], uint32_t live, int64_t at) {
@@ -154,19 +154,26 @@ __device__ __forceinline__ void copy_rows(const ghb_column& c, const T* src, con
     for (int k = 0; k < kFiltItems; k++)
       if (live >> k & 1) dst[k * kFiltThreads] = v[k];
   }
-  if (!o.is_null) return;
+  if (!o.is_null || c.type == GHB_STRING) return;
   uint8_t b[kFiltItems];
 #pragma unroll
   for (int k = 0; k < kFiltItems; k++) {
     b[k] = 0;
     if (!(live >> k & 1) || c.null_mode == GHB_NULLS_NONE) continue;
-    if (c.type == GHB_STRING) b[k] = (int32_t)((long long)v[k] & 0xffffffff) < 0;
-    else if (c.null_mode == GHB_NULLS_BYTEMAP) b[k] = c.is_null[base + rows[k]] != 0;
+    if (c.null_mode == GHB_NULLS_BYTEMAP) b[k] = c.is_null[base + rows[k]] != 0;
     else b[k] = raw_is_null(c, (int64_t)v[k], 0);
   }
 #pragma unroll
   for (int k = 0; k < kFiltItems; k++)
     if (live >> k & 1) o.is_null[at + k * kFiltThreads] = b[k];
+}
+
+// NULL map of `count` listed rows of a STRING column: a row is NULL by its pair
+// (start < 0), whatever the column's null mode.  Out of line and apart from
+// copy_rows, whose registers spill with that test (two leaves over nullable
+// columns of 40M rows: 395 us with it there, 372 apart).
+__device__ __noinline__ void string_nulls(const int2* pairs, const uint16_t* list, int count, uint8_t* is_null) {
+  for (int i = threadIdx.x; i < count; i += kFiltThreads) is_null[i] = pairs[list[i]].x < 0;
 }
 
 // Each CTA claims ranges of rows in launch order.  Per range: the predicate
@@ -313,6 +320,9 @@ __global__ void __launch_bounds__(kFiltThreads, 3) filter_kernel(const __grid_co
                                  live, out0 + i);
         }
       }
+      for (int j = 0; j < p.nproj; j++)
+        if (p.cols.c[p.proj[j]].type == GHB_STRING && p.out[j].is_null)
+          string_nulls((const int2*)p.cols.c[p.proj[j]].aux + base, list, count, p.out[j].is_null + out0);
     }
     if (r >= p.nranges) break;
     pending = r;
