@@ -56,7 +56,7 @@ __device__ __forceinline__ uint32_t small_nulls(const ghb_column& c, const int64
 }
 
 // Writes rows idx[k] (row of position pos0 + 32 k, k with bit k of `live`) of
-// column c.
+// column c (all threads of the CTA).
 template <int IT>
 __device__ __forceinline__ void small_gather(const ghb_column& c, const ghb_out_column& o, const uint32_t (&idx)[IT],
                                              int pos0, uint32_t live) {
@@ -67,7 +67,9 @@ __device__ __forceinline__ void small_gather(const ghb_column& c, const ghb_out_
     raw[k] = live >> k & 1 ? ld_raw(c, idx[k]) : 0;
     pos[k] = (uint32_t)(pos0 + 32 * k);
   }
-  put_rows<IT>(o, c.type, raw, small_nulls<IT>(c, raw, idx, live), pos, live);
+  const uint32_t nulls = small_nulls<IT>(c, raw, idx, live);
+  __syncthreads();   // the column is read whole before it is written: a column may be sorted in place
+  put_rows<IT>(o, c.type, raw, nulls, pos, live);
 }
 
 // One SM's shared-memory path bounds it (about 40 wavefronts per 32 rows and
