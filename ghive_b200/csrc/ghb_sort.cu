@@ -821,6 +821,7 @@ constexpr int kFinRounds = 2;                        // further rows read to fin
 constexpr int kFinExt = 32 + kFinRounds * kSortThreads;   // 32, then 256 a round
 constexpr int kFinNet = 16;                          // longest run one thread sorts
 constexpr int kFinField = 28;                        // key bits such a sort compares
+constexpr int kFinTieRun = 1024;                     // longest run in which a wide key's columns are compared
 
 __device__ __forceinline__ void word_order(uint32_t& a, uint32_t& b) {
   const uint32_t lo = min(a, b);
@@ -838,6 +839,30 @@ __device__ __forceinline__ void sort_words(uint32_t (&w)[kFinNet]) {
     if ((e - K % P) % (2 * K) < K && e / (2 * P) == (e + K) / (2 * P)) word_order(w[e], w[e + K]);
   if constexpr (K > 1) sort_words<N, P, K / 2>(w);
   else if constexpr (2 * P < N) sort_words<N, 2 * P, 2 * P>(w);
+}
+
+// Sorts the places src[0 .. len) by `threads` threads of a warp or a CTA (thread
+// t of them, `sync` their barrier): bitonic merges, each beginning with the
+// comparison of mirrored places, so that every comparison leaves the earlier row
+// (after(x, y): row x goes after row y) in front and places past len take no part.
+template <typename AFTER, typename SYNC>
+__device__ __forceinline__ void sort_places(uint16_t* src, int len, int t, int threads, const AFTER& after,
+                                            const SYNC& sync) {
+  for (int size = 2; size / 2 < len; size *= 2)
+    for (int stride = size / 2; stride > 0; stride /= 2) {
+      const bool mirror = stride == size / 2;
+      for (int q = t; 2 * q < len + stride; q += threads) {   // i below len
+        const int off = q & (stride - 1), i = 2 * (q - off) + off;
+        const int j = mirror ? i + size - 1 - 2 * off : i + stride;
+        if (j >= len) continue;
+        const uint16_t x = src[i], y = src[j];
+        if (after(x, y)) {
+          src[i] = y;
+          src[j] = x;
+        }
+      }
+      sync();
+    }
 }
 
 // Order of rows a and b by the whole of their keys (-1, 0, 1), for rows of a wide
@@ -883,20 +908,28 @@ __device__ __forceinline__ void sort_run(const uint32_t* s_word, uint16_t* s_src
 // The rows are sorted by their keys' bits from p.shift up; a tile puts the
 // runs that start in it (equal bits from p.shift up) in order by the lower
 // bits and writes their rows, in output order.  A run of up to kFinNet rows is
-// sorted by one thread in registers; a longer one by a warp: each row's place
-// is the number of smaller keys in the run and of equal ones before it.  A run
+// sorted by one thread in registers; one of up to 32 by a warp, a row a lane
+// that counts the rows before it; a longer one by a warp's and past kWarpRun
+// rows by the CTA's bitonic merges in shared memory.  A run
 // whose end is not found within kFinExt rows of the tile goes to the list of
 // long runs.  Bound by instruction issue (205 per 32 rows at six rows to a
 // run; DRAM 35 %): 0.54 ms for the 60M-row (d, k) sort, which it spares four
 // passes of 0.40 ms.  Other forms measured there: every row counting the rows
 // of its run before it 1.04 ms, with 64-bit keys in shared memory 0.96; one
-// list of runs found by a thread per row 0.71.
+// list of runs found by a thread per row 0.71.  A 1M-row sort of 0.18 ms with
+// one unordered run of 500 / 1000 / 2000 rows: 0.19 / 0.20 / 0.23 ms, and 0.29 /
+// 0.62 / 1.88 when a warp counted every long run; 4M rows of which 40 % lie in
+// runs of 64, 25 % in runs of 100: 0.32 and 0.33 ms (0.32 and 0.35), 0.54 and
+// 0.43 with the CTA from 33 rows on.
 template <typename V, bool WIDE>
-__global__ void __launch_bounds__(kSortThreads) sort_finish_kernel(const __grid_constant__ PassParams p) {
+__global__ void __launch_bounds__(kSortThreads, 5) sort_finish_kernel(const __grid_constant__ PassParams p) {
   constexpr int kRows = kFinTile + kFinExt;
   constexpr int kWords = kRows / 32;
   constexpr int kTileWords = kFinTile / 32;
   static_assert(kFinTile == 8 * kSortThreads && kFinTile == 2048 && kFinNet == 16, "a run's list entry");
+  // longest run a warp sorts: a longer one keeps a lone warp for too long (a
+  // comparison of a wide key's columns is a chain of loads)
+  constexpr int kWarpRun = WIDE ? 128 : 256;
   constexpr int kRuns = kFinTile / 2 + 1;        // runs of two rows and more that start in a tile
   __shared__ uint64_t s_key[kRows];
   __shared__ uint32_t s_word[kRows];             // the key's field << 4
@@ -906,6 +939,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_finish_kernel(const __grid_
   __shared__ uint16_t s_big[kRows / kFinNet];    // first rows of longer runs
   __shared__ uint32_t s_start[kWords + 1];       // bit i: row i starts a run
   __shared__ uint32_t s_n[2];                    // runs in the lists: up to 8 rows | up to kFinNet << 16; longer
+  __shared__ uint32_t s_huge;                    // some of the longer runs have more than kWarpRun rows
   if (*(volatile int32_t*)p.dev_status == kDevTimeout) return;   // the passes left invalid rows
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -925,7 +959,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_finish_kernel(const __grid_
   };
   const uint32_t fmask = (1u << min(p.shift, kFinField)) - 1u;
   if (threadIdx.x < 2) s_n[threadIdx.x] = 0;
-  if (threadIdx.x == 0) s_start[kWords] = 0;
+  if (threadIdx.x == 0) s_start[kWords] = s_huge = 0;
   // row i of the tile: its key to shared memory, and its start flag
   auto enter = [&](int i, uint64_t key) -> uint32_t {
     uint64_t prev = __shfl_up_sync(0xffffffffu, key, 1);
@@ -1021,21 +1055,26 @@ __global__ void __launch_bounds__(kSortThreads) sort_finish_kernel(const __grid_
   }
   __syncthreads();
   const int n8 = s_n[0] & 0xffffu, n16 = s_n[0] >> 16, nbig = s_n[1];
+  auto after = [&](int i, int j) -> bool { return below(j, i) || (i > j && !below(i, j)); };
   for (int m = warp; m < nbig; m += kSortThreads / 32) {
-    const int a = s_big[m], b = next_start(a);
+    const int a = s_big[m], len = next_start(a) - a;
+    if (len > kWarpRun) {
+      s_huge = 1;   // the CTA's, below
+      continue;
+    }
     bool desc = false;
-    for (int i = a + 1 + lane; i < b; i += 32) desc |= below(i, i - 1);
+    for (int i = a + 1 + lane; i < a + len; i += 32) desc |= below(i, i - 1);
     if (!__any_sync(0xffffffffu, desc)) continue;   // in order already
-    for (int i = a + lane; i < b; i += 32) {
+    if (len > 32) {
+      sort_places(s_src + a, len, lane, 32, after, [] { __syncwarp(); });
+    } else if (lane < len) {   // a row a lane: its place is the number of rows before it
+      const int i = a + lane;
       const uint64_t mine = s_key[i];
       int at = a;
-      for (int j = a; j < b; j++) {
+      for (int j = a; j < a + len; j++) {
         const uint64_t y = s_key[j];
         bool before = y < mine;
-        if (y == mine && j != i) {
-          const int o = WIDE ? row_order(p, (int64_t)vals_in[j], (int64_t)vals_in[i]) : 0;
-          before = o < 0 || (o == 0 && j < i);
-        }
+        if (y == mine && j != i) before = after(i, j);
         at += before;
       }
       s_src[at] = (uint16_t)i;
@@ -1052,6 +1091,27 @@ __global__ void __launch_bounds__(kSortThreads) sort_finish_kernel(const __grid_
     else sort_run<4>(s_word, s_src, a, len, partial, below);
   }
   __syncthreads();
+  for (int m = 0; s_huge && m < nbig; m++) {   // the longest runs, the CTA one after another
+    const int a = s_big[m], len = next_start(a) - a;
+    if (len <= kWarpRun) continue;
+    const bool whole = WIDE && len <= kFinTieRun;   // rows of equal leading bits compared by their columns
+    bool desc = false;
+    for (int i = a + 1 + threadIdx.x; i < a + len; i += kSortThreads)
+      desc |= whole ? below(i, i - 1) : s_key[i] < s_key[i - 1];
+    if (__syncthreads_or(desc))
+      sort_places(s_src + a, len, (int)threadIdx.x, kSortThreads,
+                  [&](int i, int j) {
+                    const uint64_t x = s_key[i], y = s_key[j];
+                    return x != y ? x > y : whole ? after(i, j) : i > j;
+                  },
+                  [] { __syncthreads(); });
+    // else such rows are reported when they are out of order
+    for (int i = a + 1 + threadIdx.x; WIDE && !whole && i < a + len; i += kSortThreads) {
+      const int x = s_src[i], y = s_src[i - 1];
+      if (s_key[x] == s_key[y] && row_order(p, (int64_t)vals_in[x], (int64_t)vals_in[y]) < 0)
+        *(volatile unsigned int*)p.ties = 1;
+    }
+  }
   for (int h = 0; h < kFinTile && h < end; h += kSortThreads * kFinItems) {
     V val[kFinItems];
     uint64_t x[kFinItems];
