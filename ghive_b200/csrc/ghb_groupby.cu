@@ -253,8 +253,11 @@ int32_t gb_setup(ghb_ctx* ctx, const ghb_predicate* pred, const ghb_column* cols
   // 326); INT keys (4096 / 2048) 50,000 636 / 617, 1M 836 / 679.  163 KB leaves
   // a row per thread: 1M groups 682, but with 30 % passing 391 where 225 KB
   // takes 387.  Below 32,768 groups the larger table keeps more rows: INT keys,
-  // 20,000 groups 516 / 590.
-  if (nkeys && su.tile_rows == 0 && su.nstages == 0 && S > 0 && max_groups > 32768) {
+  // 20,000 groups 516 / 590.  Only a stated number of groups tells: where the
+  // capacity or the rows stand in for it the groups may be few, and 3000 of
+  // them take 461 us with 2048 slots, 722 with 1024 (LONG keys, 90 % passing).
+  const bool stated = su.max_groups > 0 && su.max_groups < n;
+  if (nkeys && su.tile_rows == 0 && su.nstages == 0 && S > 0 && stated && max_groups > 32768) {
     const size_t cap = std::min<size_t>(smem_cap, 195 * 1024);
     int s = S, t = kGbRows * threads;
     while (t > threads && table_bytes_smem(S) + 2 * stage_bytes_of(t) > smem_cap) t /= 2;
