@@ -245,29 +245,21 @@ int32_t gb_setup(ghb_ctx* ctx, const ghb_predicate* pred, const ghb_column* cols
     while (S > 64 && table_bytes_smem(S) + 2 * stage_bytes_of(threads) > smem_cap) S /= 2;
   // Rows that go past the shared table wait for the global one, and their loads
   // and atomics in flight are held by the L1 that shared memory leaves over (28
-  // KB at 225 KB, 60 KB at 195, 92 at 163).  With many groups the CTA keeps
-  // within 195 KB, where a table halved for it (not below 1024 slots) and the
-  // tile it would have anyway fit.  Fold of 16M rows of the fact aggregates at
-  // 225 / 195 KB, 90 % of them passing: LONG keys (2048 / 1024 slots) 100,000
-  // groups 758 / 670 us, 1M 821 / 714, 50,000 685 / 690 (30 % passing: 339 /
-  // 326); INT keys (4096 / 2048) 50,000 636 / 617, 1M 836 / 679.  163 KB leaves
-  // a row per thread: 1M groups 682, but with 30 % passing 391 where 225 KB
-  // takes 387.  Below 32,768 groups the larger table keeps more rows: INT keys,
-  // 20,000 groups 516 / 590.  Only a stated number of groups tells: where the
-  // capacity or the rows stand in for it the groups may be few, and 3000 of
-  // them take 461 us with 2048 slots, 722 with 1024 (LONG keys, 90 % passing).
+  // KB at 225 KB, 60 KB at 195).  With many groups stated, the CTA keeps within
+  // 195 KB where its table and a tile of a row per thread fit.  Fold of 16M rows
+  // of the fact aggregates by LONG keys (2048 slots) at 225 / 195 KB, 90 % of
+  // them passing: 50,000 groups 809 / 702 us, 100,000 818 / 729, 300,000 826 /
+  // 781, 1M 1196 / 897; 30 % passing: 391 / 395, 393 / 395, 420 / 418, 611 /
+  // 616.  The table keeps its slots: half of them leave two rows per thread and
+  // are as fast there, but take 722 us for 3000 groups where a million were
+  // stated (490 with all, 478 at 225 KB), and so do half of the 4096 slots of INT
+  // keys, which do not fit otherwise (462 against 302).  Where the capacity or
+  // the rows stand in for the number, the groups may be few, and the larger tile
+  // is the faster one (3000 groups, 30 % passing: 369 / 399).
   const bool stated = su.max_groups > 0 && su.max_groups < n;
-  if (nkeys && su.tile_rows == 0 && su.nstages == 0 && S > 0 && stated && max_groups > 32768) {
-    const size_t cap = std::min<size_t>(smem_cap, 195 * 1024);
-    int s = S, t = kGbRows * threads;
-    while (t > threads && table_bytes_smem(S) + 2 * stage_bytes_of(t) > smem_cap) t /= 2;
-    if (su.smem_slots == 0)
-      while (s > 1024 && table_bytes_smem(s) + 2 * stage_bytes_of(t) > cap) s /= 2;
-    if (table_bytes_smem(s) + 2 * stage_bytes_of(t) <= cap) {
-      S = s;
-      smem_cap = cap;
-    }
-  }
+  if (nkeys && su.tile_rows == 0 && su.nstages == 0 && S > 0 && stated && max_groups > 32768 &&
+      table_bytes_smem(S) + 2 * stage_bytes_of(threads) <= 195 * 1024)
+    smem_cap = std::min<size_t>(smem_cap, 195 * 1024);
   reserve = std::max(S, su.smem_table_slots);
   if (table_bytes_smem(reserve) + 2 * stage_bytes_of(threads) > smem_cap)
     return set_error(ctx, GHB_ERR_UNSUPPORTED,
