@@ -453,11 +453,27 @@ static int32_t batch_create(ghb_ctx* ctx, const ghb_groupby_instance* inst, int3
   const int forced_threads =
       (cfg && (cfg->block_threads == 512 || cfg->block_threads == 1024)) ? cfg->block_threads : 0;
   const float lf = (cfg && cfg->load_factor > 0.f) ? cfg->load_factor : 0.5f;
-  // the setting of a batch that is not tuned: 24 instances of 10^4 to 4 10^6
-  // rows and 10 to 10^5 groups fold in 1.06 ms with 2048 shared slots and a load
-  // factor of 0.5 throughout, 0.86 with 1024 slots, and 0.78 with a load
-  // factor of 0.25 above 2048 groups as well (while those tables stay in 2 GB)
-  BatchSetting base{forced_threads ? forced_threads : kGbThreads, 1024, 0, lf, {0.f, 0.f, 0.f, 0.f}};
+  // The setting of a batch that is not tuned.  Shared slots: 1024 where most rows
+  // belong to instances of more groups than either table holds (the smaller one
+  // leaves L1 for what goes past it) or of no more than it holds well; 2048 where
+  // the larger table makes the difference.  16 instances of 1M rows, 90 / 30 %
+  // passing, 1024 against 2048 slots, us: 700 groups 383 / 338 against 427 / 385,
+  // 1100 groups 544 / 498 against 478 / 443, 1500 701 / 536 against 529 / 491,
+  // 2048 807 / 582 against 617 / 554, 3000 916 / 620 against 1118 / 763, 20,000
+  // 1156 / 700 against 1981 / 973; 12 of 1500 with 4 of 3000 762 / 562 against 710
+  // / 568, 8 with 8 815 / 582 against 874 / 638; 4 of 1500 with 12 of 700 461 /
+  // 387 against 450 / 410.
+  int64_t rows_small = 0, rows_mid = 0, rows_past = 0;
+  for (const InstSpec& s : spec) {
+    if (s.groups > 2048) rows_past += s.rows;
+    else if (s.groups > 1024) rows_mid += s.rows;
+    else if (s.groups > 512) rows_small += s.rows;
+  }
+  const int32_t slots = rows_mid > 0 && rows_mid >= 3 * rows_past + rows_small / 3 ? 2048 : 1024;
+  // Load factor: 0.25 above 2048 groups while those tables stay in 2 GB (24
+  // instances of 10^4 to 4 10^6 rows and 10 to 10^5 groups with 1024 slots: 0.86
+  // ms at 0.5 throughout, 0.78)
+  BatchSetting base{forced_threads ? forced_threads : kGbThreads, slots, 0, lf, {0.f, 0.f, 0.f, 0.f}};
   int64_t roomy_bytes = 0;
   for (const InstSpec& s : spec)
     if (s.groups > 2048) roomy_bytes += next_pow2_i64(4 * s.groups + 1) * 8 * (2 + 2 * naggs);
