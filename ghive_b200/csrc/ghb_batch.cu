@@ -547,6 +547,11 @@ static int32_t batch_create(ghb_ctx* ctx, const ghb_groupby_instance* inst, int3
   trials += "]";
   std::vector<GbParams> ps;
   int32_t st = plan_image(ctx, spec, sig, best, stream, &b->im, &ps);
+  if (st == GHB_ERR_OOM && !tune && best.lf_class[2] > 0.f) {   // the tables at half their slots may fit still
+    best.lf_class[2] = best.lf_class[3] = 0.f;
+    ctx->last_error.clear();
+    st = plan_image(ctx, spec, sig, best, stream, &b->im, &ps);
+  }
   if (st) return st;
 
   // report: the setting, the trials and the shared slots per size class

@@ -507,12 +507,23 @@ int32_t filter_groupby_impl(ghb_ctx* ctx, const ghb_predicate* pred, const ghb_c
     GHB_CUDA_TRY(ctx, cudaMemsetAsync(fixed_table, 0, table_bytes, stream));
     table = fixed_table;
   } else {
-    if (table_bytes > ctx->gb_bytes || ctx->gb_dirty || !ctx->gb_table) {
-      if (table_bytes > ctx->gb_bytes) {
-        int32_t gst = regrow(ctx, &ctx->gb_table, &ctx->gb_bytes, std::max(table_bytes, (size_t)1 << 20),
-                             stream, false);
-        if (gst) return gst;
-      }
+    auto grow = [&]() -> int32_t {
+      return table_bytes <= ctx->gb_bytes ? GHB_OK
+                                          : regrow(ctx, &ctx->gb_table, &ctx->gb_bytes,
+                                                   std::max(table_bytes, (size_t)1 << 20), stream, false);
+    };
+    bool fresh = table_bytes > ctx->gb_bytes || ctx->gb_dirty || !ctx->gb_table;
+    st = grow();
+    if (st == GHB_ERR_OOM && su.roomy) {   // the table at half its slots may fit still
+      su.roomy = 0;
+      ctx->last_error.clear();
+      if ((st = gb_setup(ctx, pred, cols, ncols, key_cols, nkeys, aggs, naggs, out, out_capacity, d_out_groups, su,
+                         &p, &f, &table_bytes, &smem)))
+        return st;
+      st = grow();
+    }
+    if (st) return st;
+    if (fresh) {
       GHB_CUDA_TRY(ctx, cudaMemsetAsync(ctx->gb_table, 0, ctx->gb_bytes, stream));
       ctx->gb_dirty = false;
     }
