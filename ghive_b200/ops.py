@@ -129,7 +129,10 @@ class _Outs:
     def ptr(self):
         return C.addressof(self.arr)
 
-    def rows(self, k):
+    def rows(self, k, fresh=False):
+        """The first k rows: views of the value columns, and NULL maps as bool
+        tensors of their own, or views of these when the outputs are made for one
+        call (`fresh`) and nothing writes to them again."""
         out = []
         for (d, nl), o in zip(self.cols, self.arr):
             m = 2 * k if o.type == abi.STRING else k
@@ -137,9 +140,12 @@ class _Outs:
                 d = d[:m]
             if nl is not None and len(nl) != k:
                 nl = nl[:k]
-            # the kernels write 0 or 1: a device map's bytes are a bool tensor's
-            out.append((d, None if nl is None else nl.view(torch.bool) if torch is not None and
-                        isinstance(nl, torch.Tensor) else nl.astype(bool)))
+            if nl is None:
+                out.append((d, None))
+            elif torch is None or not isinstance(nl, torch.Tensor):
+                out.append((d, nl.astype(bool)))
+            else:   # the kernels write 0 or 1: a map's bytes are a bool tensor's
+                out.append((d, nl.view(torch.bool) if fresh else nl.bool()))
         return out
 
 
@@ -285,7 +291,8 @@ class Context:
         n = cs[0].n if cs.n else 0
         proj = list(range(cs.n)) if proj is None else list(proj)
         cap = n if capacity is None else capacity
-        if outs is None:
+        fresh = outs is None
+        if fresh:
             outs = _Outs([cs[j].type for j in proj], cap, self.torch_device, with_nulls=with_nulls)
         pa = (C.c_int32 * max(1, len(proj)))(*proj)
         d_rows = torch.empty(1, dtype=torch.int64, device=self.torch_device)  # the kernel writes it
@@ -296,7 +303,7 @@ class Context:
         if not sync:
             return outs, d_rows
         k = self._sync_count(d_rows, stream)
-        return outs.rows(min(k, cap)), k
+        return outs.rows(min(k, cap), fresh), k
 
     def filter_groupby(self, pred, cols, keys, aggs, capacity=None, max_groups=None, cfg=None,
                        stream=None, sync=True):
@@ -324,7 +331,7 @@ class Context:
         if not sync:
             return outs, d_groups
         g = self._sync_count(d_groups, stream)
-        res = outs.rows(min(g, cap))
+        res = outs.rows(min(g, cap), True)
         return res[:len(keys)], res[len(keys):], g
 
     def batch_groupby(self, instances, keys, aggs, autotune=True, block_threads=0, smem_slots=0,
@@ -386,7 +393,8 @@ class Context:
         if capacity is None:
             _, dup, _ = table.info()
             capacity = max(1, n * max(1, dup))
-        if outs is None:
+        fresh = outs is None
+        if fresh:
             ob = _Outs(table.payload_types, capacity, self.torch_device)
             op = _Outs([ppl[j].type for j in range(ppl.n)], capacity, self.torch_device)
             prow = torch.empty(capacity, dtype=torch.int32, device=self.torch_device) if rowids else None
@@ -404,7 +412,7 @@ class Context:
         m = min(k, capacity)
         return {"rows": k, "probe_rowid": None if prow is None else prow[:m],
                 "build_rowid": None if brow is None else brow[:m],
-                "build": ob.rows(m), "probe": op.rows(m)}
+                "build": ob.rows(m, fresh), "probe": op.rows(m, fresh)}
 
     def sort(self, keys, orders=None, null_orders=None, payload=(), rowid=False, stream=None,
              sync=True, with_nulls=True, outs=None):
@@ -413,7 +421,8 @@ class Context:
         outputs, payload outputs) reuses output columns made earlier."""
         ks, ps = _Cols(keys), _Cols(payload)
         n = ks[0].n
-        if outs is not None:
+        fresh = outs is None
+        if not fresh:
             ok, op = outs
         else:
             ok = _Outs([ks[j].type for j in range(ks.n)], n, self.torch_device, with_nulls=with_nulls)
@@ -425,7 +434,7 @@ class Context:
                                    _ptr(rid), None, _stream(stream)))
         if sync:
             self.sync(stream)
-        return ok.rows(n), op.rows(n), (None if rid is None else rid[:n])
+        return ok.rows(n, fresh), op.rows(n, fresh), (None if rid is None else rid[:n])
 
     # -------------------------------------------------------------- host ops
     def filter_host(self, pred, cols, proj=None, capacity=None, outs=None):
