@@ -42,6 +42,7 @@ import os
 import statistics
 import subprocess
 import sys
+import tempfile
 import threading
 import time
 
@@ -654,15 +655,15 @@ def bench_sort(ctx, args, dev, stream, peak, peak_kind):
         for _ in range(max(1, args.warmup)):
             ctx.sort([dd, dk], payload=[dr], sync=False, outs=souts)
         ctx.sync()
-        l0 = ctx.launches
-        ctx.sort([dd, dk], payload=[dr], sync=False, outs=souts)
+        # the radix passes that the sort's plan came to, and whether they cover the
+        # leading digits only and a finish sorts the rest: from one call's log line
+        with tempfile.NamedTemporaryFile("r", suffix=".jsonl") as log:
+            ctx.set_log(log.name)
+            ctx.sort([dd, dk], payload=[dr], sync=False, outs=souts)
+            ctx.set_log(None)
+            plan = json.loads(log.read().splitlines()[-1])
         ctx.sync()
-        # the sort launches a min/max, a sample and a histogram kernel, then one
-        # kernel per executed radix pass; when it sorts by the leading digits
-        # alone, two finish kernels follow.  All 52 bits are seven passes.
-        kernels = ctx.launches - l0 - 3
-        finish = kernels < 7
-        passes = kernels - 2 if finish else kernels
+        passes, finish = plan["passes"], plan["finish"]
         times = []
         for _ in range(max(3, min(args.steps, 10))):
             a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

@@ -49,6 +49,10 @@ struct ghb_ctx {
   // pinned host words a sync reads back: the status word, a count
   int64_t* h_sync = nullptr;
 
+  // what the last sort's plan came to, for its log line: radix passes launched
+  // (-1: the one-CTA sort), and whether a finish sorts the rest
+  int32_t sort_passes = -1, sort_finish = 0;
+
   // self-resetting counters: [0] tile claim, [1] finished CTAs, ...
   unsigned long long* d_counters = nullptr;
 

@@ -6,7 +6,9 @@
 // line per call in that file:
 //   level 1: {"op", "device", "rows", "bytes", "host_us", "status"}: host_us is
 //            the call's own time (the enqueue of an asynchronous call, the
-//            whole call for the host-buffer and plan entry points);
+//            whole call for the host-buffer and plan entry points); a sort
+//            adds "passes", the radix passes it launched, and "finish", 1 when
+//            they covered the leading digits only;
 //   level 2: an asynchronous call is also bracketed by CUDA events on its
 //            stream and waits for them, adding "device_us", "gbs" (bytes /
 //            device_us) and, when the log was given a peak, "roofline_frac";
@@ -53,6 +55,10 @@ class CallScope {
   CallScope& operator=(const CallScope&) = delete;
   void rows(int64_t r) { rows_ = r; }
   void bytes(int64_t b) { bytes_ = b; }
+  void passes(int32_t n, int32_t finish) {
+    passes_ = n;
+    finish_ = finish;
+  }
   int32_t done(int32_t st) {
     status_ = st;
     return st;
@@ -77,6 +83,7 @@ class CallScope {
       std::fprintf(ctx_->log, ", \"device_us\": %.1f, \"gbs\": %.6g", dev_us, gbs);
       if (ctx_->log_peak_gbs > 0) std::fprintf(ctx_->log, ", \"roofline_frac\": %.6g", gbs / ctx_->log_peak_gbs);
     }
+    if (passes_ >= 0) std::fprintf(ctx_->log, ", \"passes\": %d, \"finish\": %d", passes_, finish_);
     std::fprintf(ctx_->log, ", \"status\": %d}\n", status_);
   }
 
@@ -87,6 +94,7 @@ class CallScope {
   std::chrono::steady_clock::time_point t0_{};
   bool timed_ = false;
   int64_t rows_ = 0, bytes_ = 0;
+  int32_t passes_ = -1, finish_ = 0;
   int32_t status_ = GHB_OK;
 };
 

@@ -1319,6 +1319,8 @@ static int32_t run_passes(ghb_ctx* ctx, PassParams& pp, const std::vector<Segmen
   const bool finish = shift0 > 0;   // the passes leave the lower bits to the finish
   int total = 0;
   for (auto& r : run) total += (int)r.size();
+  ctx->sort_passes = total;
+  ctx->sort_finish = finish;
   const int64_t n = pp.n;
   V* vb[2] = {(V*)vbv[0], (V*)vbv[1]};
   const bool multi = segs.size() > 1;
@@ -1820,9 +1822,13 @@ extern "C" int32_t ghb_sort(ghb_ctx* ctx, const ghb_column* keys, const int32_t*
   const size_t extra = strings ? string_sort_scratch_bytes(keys, nkeys, n) : 0;
   int32_t st = scratch_reserve(ctx, sort_scratch_bytes(n) + extra, (cudaStream_t)stream);
   if (st) return cs.done(st);
+  ctx->sort_passes = -1;
   if (strings)
-    return cs.done(sort_with_strings(ctx, keys, orders, null_orders, nkeys, payload, npayload, out_keys,
-                                     out_payload, out_rowid, cfg, (cudaStream_t)stream));
-  return cs.done(sort_impl(ctx, keys, orders, null_orders, nkeys, payload, npayload, out_keys, out_payload,
-                           out_rowid, cfg, (cudaStream_t)stream));
+    st = sort_with_strings(ctx, keys, orders, null_orders, nkeys, payload, npayload, out_keys, out_payload, out_rowid,
+                           cfg, (cudaStream_t)stream);
+  else
+    st = sort_impl(ctx, keys, orders, null_orders, nkeys, payload, npayload, out_keys, out_payload, out_rowid, cfg,
+                   (cudaStream_t)stream);
+  cs.passes(ctx->sort_passes, ctx->sort_finish);
+  return cs.done(st);
 }
