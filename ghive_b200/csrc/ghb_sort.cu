@@ -1275,38 +1275,40 @@ size_t sort_scratch_bytes(int64_t n) {
   return b + 4096;
 }
 
+// The forms of the pass over V values that a sort uses: a 64-bit value is a lone
+// payload, carried by a one-segment key, which is always packed and decoded; a
+// key of several segments carries the 32-bit row index, reads the columns at
+// first and gathers at last.
+#define GHB_EACH_PASS(DO)           \
+  do {                              \
+    DO(kSrcPacked, kDstPacked);     \
+    DO(kSrcPacked, kDstDecode);     \
+    if constexpr (sizeof(V) == 4) { \
+      DO(kSrcPacked, kDstGather);   \
+      DO(kSrcCols, kDstPacked);     \
+      DO(kSrcCols, kDstGather);     \
+      DO(kSrcPerm, kDstPacked);     \
+      DO(kSrcPerm, kDstGather);     \
+    }                               \
+  } while (0)
+
 template <typename V>
 static void launch_pass(int src, int dst, int grid, size_t dyn, cudaStream_t s, const PassParams& pp) {
-#define GHB_PASS(S, D) sort_pass_kernel<V, S, D><<<grid, kSortThreads, dyn, s>>>(pp)
-  if (src == kSrcPacked && dst == kDstPacked) GHB_PASS(kSrcPacked, kDstPacked);
-  else if (src == kSrcPacked && dst == kDstDecode) GHB_PASS(kSrcPacked, kDstDecode);
-  else if (src == kSrcPacked && dst == kDstGather) GHB_PASS(kSrcPacked, kDstGather);
-  else if (src == kSrcCols && dst == kDstPacked) GHB_PASS(kSrcCols, kDstPacked);
-  else if (src == kSrcCols && dst == kDstDecode) GHB_PASS(kSrcCols, kDstDecode);
-  else if (src == kSrcCols && dst == kDstGather) GHB_PASS(kSrcCols, kDstGather);
-  else if (src == kSrcPerm && dst == kDstPacked) GHB_PASS(kSrcPerm, kDstPacked);
-  else if (src == kSrcPerm && dst == kDstGather) GHB_PASS(kSrcPerm, kDstGather);
+#define GHB_PASS(S, D) \
+  if (src == S && dst == D) sort_pass_kernel<V, S, D><<<grid, kSortThreads, dyn, s>>>(pp)
+  GHB_EACH_PASS(GHB_PASS);
 #undef GHB_PASS
 }
 
 template <typename V>
 static int32_t set_smem(ghb_ctx* ctx, size_t dyn) {
 #define GHB_ATTR(S, D) \
-  do {                                                                      \
-    int32_t _st = ensure_dyn_smem(ctx, (const void*)sort_pass_kernel<V, S, D>, dyn); \
-    if (_st) return _st;                                                    \
-  } while (0)
-  GHB_ATTR(kSrcPacked, kDstPacked);
-  GHB_ATTR(kSrcPacked, kDstDecode);
-  GHB_ATTR(kSrcPacked, kDstGather);
-  GHB_ATTR(kSrcCols, kDstPacked);
-  GHB_ATTR(kSrcCols, kDstDecode);
-  GHB_ATTR(kSrcCols, kDstGather);
-  GHB_ATTR(kSrcPerm, kDstPacked);
-  GHB_ATTR(kSrcPerm, kDstGather);
+  if (int32_t st = ensure_dyn_smem(ctx, (const void*)sort_pass_kernel<V, S, D>, dyn)) return st
+  GHB_EACH_PASS(GHB_ATTR);
 #undef GHB_ATTR
   return GHB_OK;
 }
+#undef GHB_EACH_PASS
 
 // kb / vb: key and value ping-pong buffers; packed: kb[0] / vb[0] already
 // hold the packed keys and values of a one-segment key.
@@ -1369,12 +1371,18 @@ static int32_t run_passes(ghb_ctx* ctx, PassParams& pp, const std::vector<Segmen
     pp.vals_out = vb[cur ^ 1];
     pp.shift = shift0;
     const int fgrid = (int)((n + kFinTile - 1) / kFinTile);
-    if (pp.wide) sort_finish_kernel<V, true><<<fgrid, kSortThreads, 0, stream>>>(pp);
-    else sort_finish_kernel<V, false><<<fgrid, kSortThreads, 0, stream>>>(pp);
-    GHB_LAUNCH_CHECK(ctx);
     const int lgrid = (int)std::min<int64_t>(n / kFinTile + 1, ctx->num_sms);
-    if (pp.wide) sort_finish_long_kernel<V, true><<<lgrid, kLongThreads, 0, stream>>>(pp);
-    else sort_finish_long_kernel<V, false><<<lgrid, kLongThreads, 0, stream>>>(pp);
+    if constexpr (sizeof(V) == 4)   // a wide key carries the row index
+      if (pp.wide) {
+        sort_finish_kernel<V, true><<<fgrid, kSortThreads, 0, stream>>>(pp);
+        GHB_LAUNCH_CHECK(ctx);
+        sort_finish_long_kernel<V, true><<<lgrid, kLongThreads, 0, stream>>>(pp);
+        GHB_LAUNCH_CHECK(ctx);
+        return GHB_OK;
+      }
+    sort_finish_kernel<V, false><<<fgrid, kSortThreads, 0, stream>>>(pp);
+    GHB_LAUNCH_CHECK(ctx);
+    sort_finish_long_kernel<V, false><<<lgrid, kLongThreads, 0, stream>>>(pp);
     GHB_LAUNCH_CHECK(ctx);
   }
   return GHB_OK;
