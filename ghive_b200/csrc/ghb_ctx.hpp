@@ -59,6 +59,7 @@ struct ghb_ctx {
   // group-by global table, zeroed after each finalize
   void* gb_table = nullptr;
   size_t gb_bytes = 0;
+  size_t gb_denied = ~(size_t)0;   // the smallest table that could not be allocated and had a smaller one in its place
   bool gb_dirty = false;
 
   // pinned staging for the host-buffer entry points

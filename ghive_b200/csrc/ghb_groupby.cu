@@ -512,14 +512,21 @@ int32_t filter_groupby_impl(ghb_ctx* ctx, const ghb_predicate* pred, const ghb_c
                                           : regrow(ctx, &ctx->gb_table, &ctx->gb_bytes,
                                                    std::max(table_bytes, (size_t)1 << 20), stream, false);
     };
+    auto halve = [&]() -> int32_t {   // the table at a load factor of 0.5
+      su.roomy = 0;
+      return gb_setup(ctx, pred, cols, ncols, key_cols, nkeys, aggs, naggs, out, out_capacity, d_out_groups, su, &p,
+                      &f, &table_bytes, &smem);
+    };
+    // a size that this context was refused before is not tried again: the try frees
+    // the smaller table first
+    if (su.roomy && table_bytes > ctx->gb_bytes && table_bytes >= ctx->gb_denied && (st = halve())) return st;
     bool fresh = table_bytes > ctx->gb_bytes || ctx->gb_dirty || !ctx->gb_table;
     st = grow();
-    if (st == GHB_ERR_OOM && su.roomy) {   // the table at half its slots may fit still
-      su.roomy = 0;
+    if (st == GHB_ERR_OOM && su.roomy) {
+      ctx->gb_denied = std::min(ctx->gb_denied, table_bytes);
       ctx->last_error.clear();
-      if ((st = gb_setup(ctx, pred, cols, ncols, key_cols, nkeys, aggs, naggs, out, out_capacity, d_out_groups, su,
-                         &p, &f, &table_bytes, &smem)))
-        return st;
+      if ((st = halve())) return st;
+      fresh = true;
       st = grow();
     }
     if (st) return st;
