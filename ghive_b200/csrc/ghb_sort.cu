@@ -381,6 +381,7 @@ struct PassParams {
   uint32_t* status_next;       // the next pass's, zeroed by this one (nullptr: the last pass)
   unsigned long long* counters;
   int32_t* dev_status;
+  unsigned int* gave_up;       // 1: a look-back of this sort gave up, what its passes wrote is not to be used
   int32_t spin_limit;          // look-back polls before GHB_ERR_TIMEOUT
   // a key wider than 64 bits sorted by its leading 64 (the finish): rows equal in
   // those are compared by their columns, the key columns are gathered by row,
@@ -454,10 +455,11 @@ __device__ __forceinline__ uint32_t tile_load(const uint32_t* p) {
 
 // Rows of digit d in the tiles before `tile`: kTileWindow words are loaded
 // together, so a walk over many unfinished tiles pays one L2 round trip per
-// window and not per tile.  Gives up after `spin_limit` windows that brought
+// window and not per tile.  Gives up after `p.spin_limit` windows that brought
 // nothing new (GHB_ERR_TIMEOUT; the count so far, no larger than the true one).
-__device__ __forceinline__ uint32_t tile_lookback(const uint32_t* words, int64_t tile, int d, int32_t* dev_status,
-                                                  int spin_limit) {
+// That is told by the sort's own word as well: the status word keeps the first
+// error, which may be that of a call before.
+__device__ __forceinline__ uint32_t tile_lookback(const uint32_t* words, int64_t tile, int d, const PassParams& p) {
   uint32_t excl = 0;
   int64_t t = tile - 1;
   int spins = 0;
@@ -480,8 +482,9 @@ __device__ __forceinline__ uint32_t tile_lookback(const uint32_t* words, int64_t
     }
     if (found) break;
     t -= used;
-    if (used == 0 && ++spins >= spin_limit) {
-      raise_status(dev_status, kDevTimeout);
+    if (used == 0 && ++spins >= p.spin_limit) {
+      raise_status(p.dev_status, kDevTimeout);
+      *(volatile unsigned int*)p.gave_up = 1;
       break;
     }
   }
@@ -544,7 +547,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) sort_pass_kernel(const __grid
       // a look-back of this sort that gave up left this pass's input invalid
       // (rows at wrong places, some never written): claim no more tiles, so no
       // key or row index read from that input addresses anything
-      if (*(volatile int32_t*)p.dev_status == kDevTimeout) t = p.ntiles;
+      if (*(volatile unsigned int*)p.gave_up) t = p.ntiles;
       s_tile = t;
       // the tile about one round of claims ahead starts toward L2, so the
       // CTA that claims it finds its keys and values there
@@ -657,7 +660,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) sort_pass_kernel(const __grid
     // that more of them have published), then publish the prefix
     uint32_t excl = 0;
     if (tile > 0) {
-      excl = tile_lookback(p.status, tile, d, p.dev_status, p.spin_limit);
+      excl = tile_lookback(p.status, tile, d, p);
       tile_store(words, kTilePrefix | (excl + mine));
     }
     s_gb[d] = s_base[d] + excl - bexcl;
@@ -940,7 +943,7 @@ __global__ void __launch_bounds__(kSortThreads, 5) sort_finish_kernel(const __gr
   __shared__ uint32_t s_start[kWords + 1];       // bit i: row i starts a run
   __shared__ uint32_t s_n[2];                    // runs in the lists: up to 8 rows | up to kFinNet << 16; longer
   __shared__ uint32_t s_huge;                    // some of the longer runs have more than kWarpRun rows
-  if (*(volatile int32_t*)p.dev_status == kDevTimeout) return;   // the passes left invalid rows
+  if (*(volatile unsigned int*)p.gave_up) return;   // the passes left invalid rows
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int64_t t0 = (int64_t)blockIdx.x * kFinTile;
@@ -1146,7 +1149,7 @@ __global__ void __launch_bounds__(kLongThreads) sort_finish_long_kernel(const __
   __shared__ uint32_t s_hist[kBins], s_base[kBins];
   __shared__ uint16_t s_wcnt[kLongThreads / 32][kBins];
   __shared__ int64_t s_end;
-  if (*(volatile int32_t*)p.dev_status == kDevTimeout) return;
+  if (*(volatile unsigned int*)p.gave_up) return;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const uint32_t count = *(volatile uint32_t*)p.long_runs;
@@ -1258,7 +1261,10 @@ __global__ void sort_identity_kernel(PassParams p, const V* perm) {
 
 // Words of the analysis: three per key, then the sample's pair counts.
 constexpr int kStatWords = 3 * kMaxSortKeys + 9;
-constexpr int kTieWord = kStatWords;   // after them: a wide key's long run is out of order below its leading 64 bits
+// after them: a wide key's long run is out of order below its leading 64 bits; a
+// look-back gave up
+constexpr int kTieWord = kStatWords, kGaveUpWord = kStatWords + 1;
+constexpr size_t kStatBytes = (kStatWords + 2) * 8;
 
 static inline size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
@@ -1270,7 +1276,7 @@ size_t sort_scratch_bytes(int64_t n) {
   b += 2 * align256((size_t)n * 8);                        // values ping-pong
   b += 2 * align256((size_t)ntiles * kBins * 4);           // look-back words of two passes
   b += align256((size_t)kMaxSeg * kMaxPasses * kBins * 4); // histograms
-  b += align256((kStatWords + 1) * 8);                     // min/max, sample, ties
+  b += align256(kStatBytes);                               // min/max, sample, flags
   b += align256(((size_t)n / kFinTile + 2) * 4);           // long runs
   return b + 4096;
 }
@@ -1496,7 +1502,7 @@ int32_t sort_impl(ghb_ctx* ctx, const ghb_column* keys, const int32_t* orders,
     return sort_small(ctx, K, payload, npayload, out_keys, out_payload, out_rowid, n, stream);
   // one zeroed block: the analysis, the histograms, the count of long runs
   unsigned long long* d_mm = nullptr;
-  const size_t stat_bytes = align256((kStatWords + 1) * 8), hist_bytes = (size_t)kMaxSeg * kMaxPasses * kBins * 4;
+  const size_t stat_bytes = align256(kStatBytes), hist_bytes = (size_t)kMaxSeg * kMaxPasses * kBins * 4;
   if ((st = scratch_alloc(ctx, stat_bytes + hist_bytes + align256(((size_t)n / kFinTile + 2) * 4), (void**)&d_mm,
                           stream)))
     return st;
@@ -1590,6 +1596,7 @@ int32_t sort_impl(ghb_ctx* ctx, const ghb_column* keys, const int32_t* orders,
   pp.ntiles = (n + kSortTile - 1) / kSortTile;
   pp.counters = ctx->d_counters + 2;
   pp.dev_status = ctx->d_status;
+  pp.gave_up = (unsigned int*)(d_mm + kGaveUpWord);
   pp.spin_limit = ctx->spin_limit;
   pp.long_runs = d_long;
   // the leading digits alone, when the finish is to sort the rest
