@@ -28,7 +28,7 @@ constexpr int kFiltWarps = kFiltThreads / 32;
 constexpr int kFiltWords = kFiltItems * kFiltWarps;   // ballot words of one tile
 constexpr int kFiltMaxTiles = 4;                      // tiles of one claimed range
 constexpr int kMaxProj = kMaxCols;
-constexpr int kFiltEagerPolls = 64;                   // a smaller look-back bound is not put off
+constexpr int kFiltEagerPolls = 2;                    // a smaller look-back bound is not put off
 constexpr uint64_t kNotWalked = ~0ull;                // a range whose look-back is still to come
 
 // How a leaf is evaluated.  An integer column against integer literals is a
@@ -260,8 +260,9 @@ __global__ void __launch_bounds__(kFiltThreads, 3) filter_kernel(const __grid_co
     }
     if (warp == 0) {
       if (lane == 0) lookback_publish(p.lb, p.epoch, r, total);
-      // a bound this small is set to run out: it is spent here, where the
-      // earlier ranges are still at work, and not after the next range
+      // a bound of one poll is set to run out: it is spent here, where the earlier
+      // ranges are still at work, and not after the next range, when they have
+      // published (20M rows: 200 of 200 calls run out here, none there)
       uint64_t ex = kNotWalked;
       if (p.spin_limit < kFiltEagerPolls) {
         __syncwarp();
