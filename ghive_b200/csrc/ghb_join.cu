@@ -598,18 +598,18 @@ __device__ __forceinline__ void put_words(const ghb_out_column& o, int type, con
 }
 
 // Writes IT output rows of a thread (k with bit k of `live`) at wpos + pos[k]:
-// probe row row0 + 32 k with build row brow[k] (bit k of `hit`; else an outer
-// miss or a semi join's row), whose inline payload words are w[k] when INL.
-// One column at a time, its loads issued before its stores.
-template <int IT, bool INL>
+// probe row row(k) with build row brow[k] (bit k of `hit`; else an outer miss or
+// a semi join's row), whose inline payload words are w[k] when INL.  One column
+// at a time, its loads issued before its stores.
+template <int IT, bool INL, typename ROW>
 __device__ __forceinline__ void emit_rows(const EmitDesc& d, int n_inline, uint32_t live, uint32_t hit, int64_t wpos,
-                                          const int64_t (&pos)[IT], int64_t row0, const int32_t (&brow)[IT],
+                                          const int64_t (&pos)[IT], const ROW& row, const int32_t (&brow)[IT],
                                           const ulonglong2 (&w)[IT]) {
   int64_t raw[IT];
   if (d.out_prow) {
 #pragma unroll
     for (int k = 0; k < IT; k++)
-      if (live >> k & 1) __stcs(d.out_prow + wpos + pos[k], (int)row0 + k * 32 + d.prow_base);
+      if (live >> k & 1) __stcs(d.out_prow + wpos + pos[k], (int)row(k) + d.prow_base);
   }
   if (d.out_brow) {
 #pragma unroll
@@ -636,12 +636,12 @@ __device__ __forceinline__ void emit_rows(const EmitDesc& d, int n_inline, uint3
   for (int j = 0; j < d.npp; j++) {
     const ghb_column& col = d.ppay[j];
 #pragma unroll
-    for (int k = 0; k < IT; k++) raw[k] = live >> k & 1 ? ld_raw(col, row0 + k * 32) : 0;
+    for (int k = 0; k < IT; k++) raw[k] = live >> k & 1 ? ld_raw(col, row(k)) : 0;
     uint32_t nulls = 0;
     if (col.null_mode != GHB_NULLS_NONE) {
 #pragma unroll
       for (int k = 0; k < IT; k++)
-        if (live >> k & 1) nulls |= (raw_is_null(col, raw[k], row0 + k * 32) ? 1u : 0u) << k;
+        if (live >> k & 1) nulls |= (raw_is_null(col, raw[k], row(k)) ? 1u : 0u) << k;
     }
     put_words<IT>(d.opp[j], col.type, raw, nulls, wpos, pos, live);
   }
@@ -729,6 +729,22 @@ __global__ void __launch_bounds__(kJThreads, 5) join_write_lean_kernel(const __g
   }
 }
 
+// Many output rows to a probe row: join_write_many_kernel writes them.  From two
+// on, or from four without payloads, where there is little to write.  8M probe rows
+// of 400k build rows, every key 2 / 3 / 4 times (1.8 / 2.7 / 3.6 output rows to a
+// probe row), one probe and two build payloads: 626 / 965 / 1465 us by the general
+// pass, - / 780 / 878 by this one; row ids alone 198 / 253 / 326 against - / 334 /
+// 352; 5M rows of 1000, every key 8 times, row ids alone: 460 against 256.  The
+// capacity bounds the output rows, so a call that cannot have as many does not
+// launch it (4 us).
+__host__ __device__ __forceinline__ int join_many_rows(const ProbeParams& p) { return p.nbp + p.npp > 0 ? 2 : 4; }
+__host__ __device__ __forceinline__ bool join_may_be_many(const ProbeParams& p) {
+  return p.cap / join_many_rows(p) >= p.n;
+}
+__device__ __forceinline__ bool join_many(const ProbeParams& p) {
+  return join_may_be_many(p) && *p.d_out_rows >= join_many_rows(p) * p.n;
+}
+
 constexpr int kFewChains = 4;    // chains of a warp at most that it walks one after another
 constexpr int kLongChain = 16;   // further rows of a chain that is worth it
 
@@ -750,9 +766,10 @@ constexpr int kLongChain = 16;   // further rows of a chain that is worth it
 // pass on 60M rows (634-687 us against 90 + 16 + 455): the barriers, claims and
 // look-backs of a range cost more than reading the keys again.
 template <int TH, int IT>
-__global__ void __launch_bounds__(TH, 1024 / TH) join_write_kernel(const __grid_constant__ ProbeParams p) {
+__global__ void __launch_bounds__(TH, TH == 128 ? 4 : 1024 / TH) join_write_kernel(const __grid_constant__ ProbeParams p) {
   static_assert(TH * IT == kChunk, "a CTA iteration covers one chunk");
   if (p.lean && p.out_brow == nullptr && p.stats[1] <= 1) return;   // join_write_lean_kernel's case
+  if (join_many(p)) return;                                         // join_write_many_kernel's
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const bool unique = p.stats[1] <= 1;
@@ -829,7 +846,8 @@ __global__ void __launch_bounds__(TH, 1024 / TH) join_write_kernel(const __grid_
     hit &= live;
 #pragma unroll
     for (int k = 0; k < IT; k++) first[k]--;   // the build row
-    emit_rows<IT, true>(s_desc, p.n_inline, live, hit, wpos, pos, row0, first, w);
+    auto item = [&](int k) -> int64_t { return row0 + k * 32; };
+    emit_rows<IT, true>(s_desc, p.n_inline, live, hit, wpos, pos, item, first, w);
     if (unique) continue;
     // the further build rows of the threads' keys, a row of each chain a round
     uint32_t more = 0;
@@ -875,7 +893,7 @@ __global__ void __launch_bounds__(TH, 1024 / TH) join_write_kernel(const __grid_
           const int64_t here[1] = {at + done + lane};
           const ulonglong2 none[1] = {};
           const uint32_t mine = lane < m ? 1u : 0u;
-          emit_rows<1, false>(s_desc, p.n_inline, mine, mine, 0, here, row, one, none);
+          emit_rows<1, false>(s_desc, p.n_inline, mine, mine, 0, here, [&](int) -> int64_t { return row; }, one, none);
         }
         if (lane == src) more &= ~(1u << k0);
         chains--;
@@ -889,10 +907,115 @@ __global__ void __launch_bounds__(TH, 1024 / TH) join_write_kernel(const __grid_
         on |= (more >> k & 1 && j + 1 < mult[k] ? 1u : 0u) << k;
         next[k] = on >> k & 1 ? p.next_p1[first[k]] : 0;
       }
-      emit_rows<IT, false>(s_desc, p.n_inline, more, more, wpos, pos, row0, first, w);
+      emit_rows<IT, false>(s_desc, p.n_inline, more, more, wpos, pos, item, first, w);
 #pragma unroll
       for (int k = 0; k < IT; k++) first[k] = next[k] - 1;
       more = on;
+    }
+  }
+}
+
+constexpr int kManyTile = 256;   // output rows a warp puts in order at a time
+constexpr int kManyStep = 3;     // of each key, as a power of two, when 32 keys have that many
+
+// The write pass where build rows are many to a probe row.  A warp takes 32 probe
+// rows, a lane each; every lane walks its key's chain for eight build rows
+// (up to 32 when few chains are left) and lists them in shared memory, and the
+// warp writes the listed rows side by side, so that the rows of a key fill whole
+// sectors of the output columns.  UNIT: the probe rows of one count.
+//
+// 2M probe rows of 100,000 build rows, every key 16 times (29M output rows): 0.42
+// ms with one build payload, 0.83 with two of them and two of the probe's, NULL maps
+// among them.  By the general pass, whose rounds write one row of 128 keys each, a
+// part of as many sectors per column, 1.59 and 3.94 ms (1.02 and 3.05 when each
+// thread wrote one key's rows at a time).  Four rows of each key at a time instead of
+// eight: the same.
+template <int UNIT>
+__global__ void __launch_bounds__(kJThreads, 4) join_write_many_kernel(const __grid_constant__ ProbeParams p) {
+  if (!join_many(p)) return;
+  constexpr int kIt = UNIT / 32, kWarps = kJThreads / 32;
+  __shared__ EmitDesc s_desc;
+  __shared__ int32_t s_brow[kWarps][kManyTile];   // listed build rows (-1: none), a chain's together
+  __shared__ int64_t s_pos[kWarps][32];           // per chain: output row of its first listed
+  __shared__ int32_t s_cnt[kWarps][32];           // listed rows
+  __shared__ uint8_t s_lane[kWarps][32];          // probe row
+  load_emit_desc(p, &s_desc);
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  int32_t* brow = s_brow[warp];
+  const int64_t nwork = (p.n + 31) / 32;
+  for (int64_t q = (int64_t)blockIdx.x * kWarps + warp; q < nwork; q += (int64_t)gridDim.x * kWarps) {
+    // the unit's rows up to this one's 32: their output rows come before
+    const int64_t unit = q / kIt;
+    const int item = (int)(q % kIt);
+    int64_t pos = p.chunk_count[unit], before = 0;
+    int32_t slot = -1, left = 0, cur = 0;   // cur: build row + 1, 0 none
+#pragma unroll
+    for (int k = 0; k < kIt; k++) {
+      if (k > item) break;
+      const int64_t row = unit * UNIT + k * 32 + lane;
+      const int32_t s = row < p.n ? p.slot_of_row[row] : -2;
+      slot = s >= 0 ? s & ~p.dup_bit : s;
+      int2 m = make_int2(0, 0);
+      if (s >= 0 && (k == item || p.dup_bit == 0 || (s & p.dup_bit))) m = p.meta[slot];
+      else if (s >= 0) m.y = 1;
+      if (k < item) before += s != -2 ? out_rows_of(p.join_type, m.y) : 0;
+      left = s != -2 ? out_rows_of(p.join_type, m.y) : 0;
+      cur = m.x;
+    }
+    int64_t incl = left;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t t = __shfl_up_sync(0xffffffffu, (long long)incl, o);
+      before += __shfl_xor_sync(0xffffffffu, (long long)before, o);
+      if (lane >= o) incl += t;
+    }
+    pos += before + incl - left;
+    const int64_t row0 = unit * UNIT + item * 32;
+    while (true) {
+      const unsigned act = __ballot_sync(0xffffffffu, left > 0);
+      if (!act) break;
+      const int longest = __reduce_max_sync(0xffffffffu, left);
+      const int chains = __popc(act);
+      int sh = kManyStep;   // rows listed of a chain, as a power of two
+      while (sh > 0 && longest <= 1 << (sh - 1)) sh--;
+      while (sh < 5 && longest > 1 << sh && chains << (sh + 1) <= kManyTile) sh++;
+      if (left > 0) {
+        const int r = __popc(act & lt), cnt = min(1 << sh, left);
+        s_pos[warp][r] = pos;
+        s_cnt[warp][r] = cnt;
+        s_lane[warp][r] = (uint8_t)lane;
+        for (int i = 0; i < cnt; i++) {
+          brow[(r << sh) + i] = cur - 1;
+          if (--left > 0) {
+            cur = slot >= 0 ? p.chain_p1[slot] : p.next_p1[cur - 1];
+            slot = -1;   // the chain's head is taken once
+          }
+        }
+        pos += cnt;
+      }
+      __syncwarp();
+      for (int e = lane; e < chains << sh; e += 128) {
+        int32_t b[4], f[4];
+        int64_t at[4];
+        const ulonglong2 none[4] = {};
+        uint32_t in = 0, hit = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int x = e + 32 * k, r = x >> sh, i = x & ((1 << sh) - 1);
+          const bool mine = x < chains << sh && i < s_cnt[warp][r];
+          b[k] = mine ? brow[x] : -1;
+          at[k] = mine ? s_pos[warp][r] + i : 0;
+          f[k] = mine ? s_lane[warp][r] : 0;
+          if (mine && at[k] >= p.cap) raise_status(p.status, kDevCapacity);
+          else in |= (mine ? 1u : 0u) << k;
+          hit |= (b[k] >= 0 ? 1u : 0u) << k;
+        }
+        emit_rows<4, false>(s_desc, p.n_inline, in, hit & in, 0, at, [&](int k) -> int64_t { return row0 + f[k]; }, b,
+                            none);
+      }
+      __syncwarp();   // the lists are the next rows'
     }
   }
 }
@@ -1135,13 +1258,15 @@ int32_t join_probe_impl(ghb_ctx* ctx, const ghb_join_table* t, const ghb_column*
   void (*write_kernel)(ProbeParams) = nullptr;
   void (*write_lean)(ProbeParams) = nullptr;
   void (*count_direct)(ProbeParams) = nullptr;
+  void (*write_many)(ProbeParams) = nullptr;
 #define GHB_COUNT(TH, IT)                                                                   \
   count_kernel = kint ? (knull ? join_count_kernel<TH, IT, true, true> : join_count_kernel<TH, IT, true, false>) \
                       : (knull ? join_count_kernel<TH, IT, false, true> : join_count_kernel<TH, IT, false, false>); \
   count_direct = kint ? (knull ? join_count_direct_kernel<TH, IT, true, true> : join_count_direct_kernel<TH, IT, true, false>) \
                       : (knull ? join_count_direct_kernel<TH, IT, false, true> : join_count_direct_kernel<TH, IT, false, false>); \
   write_kernel = join_write_kernel<TH, IT>;                                                  \
-  write_lean = join_write_lean_kernel<32 * IT>
+  write_lean = join_write_lean_kernel<32 * IT>;                                              \
+  write_many = join_write_many_kernel<32 * IT>
   if (threads == 128) { GHB_COUNT(128, 8); }
   else if (threads == 512) { GHB_COUNT(512, 2); }
   else { GHB_COUNT(256, 4); }
@@ -1162,6 +1287,12 @@ int32_t join_probe_impl(ghb_ctx* ctx, const ghb_join_table* t, const ghb_column*
   grid = (int)std::min<int64_t>(p.nchunks, (int64_t)ctx->num_sms * std::max(1, per_sm));
   write_kernel<<<grid, threads, 0, stream>>>(p);
   GHB_LAUNCH_CHECK(ctx);
+  if (join_may_be_many(p)) {   // the write pass of many build rows to a probe row, when the count pass finds them
+    if ((st = resident_ctas(ctx, (const void*)write_many, kJThreads, 0, &per_sm))) return st;
+    grid = (int)std::min<int64_t>((p.n + kJThreads - 1) / kJThreads, (int64_t)ctx->num_sms * std::max(1, per_sm));
+    write_many<<<grid, kJThreads, 0, stream>>>(p);
+    GHB_LAUNCH_CHECK(ctx);
+  }
   if (p.lean && !p.out_brow) {   // the lean write pass, when the build's keys turn out unique
     if ((st = resident_ctas(ctx, (const void*)write_lean, kJThreads, 0, &per_sm))) return st;
     grid = (int)std::min<int64_t>((nunits * 32 + kJThreads - 1) / kJThreads, (int64_t)ctx->num_sms * std::max(1, per_sm));
