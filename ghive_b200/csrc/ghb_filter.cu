@@ -187,7 +187,7 @@ __device__ __noinline__ void string_nulls(const int2* pairs, const uint16_t* lis
 // takes references into them, which would otherwise copy the whole parameter
 // block to every thread's stack.
 //
-// Bound by the latency of its loads at three CTAs per SM (80 registers; DRAM
+// Bound by the latency of its loads at three CTAs per SM (78 registers; DRAM
 // 42-50 % busy).  One B200, before (a row's whole tree interpreted at a time,
 // one range at a time) and now: d < cut on 6M rows, half pass, 71 -> 48 us;
 // the same on 40M rows 400 -> 300 us; two leaves over nullable columns, 6 % of

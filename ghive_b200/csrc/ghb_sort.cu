@@ -916,7 +916,7 @@ __device__ __forceinline__ void sort_run(const uint32_t* s_word, uint16_t* s_src
 // rows by the CTA's bitonic merges in shared memory.  A run
 // whose end is not found within kFinExt rows of the tile goes to the list of
 // long runs.  Bound by instruction issue (205 per 32 rows at six rows to a
-// run; DRAM 35 %): 0.54 ms for the 60M-row (d, k) sort, which it spares four
+// run; DRAM 35 %): 0.56 ms for the 60M-row (d, k) sort, which it spares four
 // passes of 0.40 ms.  Other forms measured there: every row counting the rows
 // of its run before it 1.04 ms, with 64-bit keys in shared memory 0.96; one
 // list of runs found by a thread per row 0.71.  A 1M-row sort of 0.18 ms with
@@ -1399,7 +1399,7 @@ static int32_t run_passes(ghb_ctx* ctx, PassParams& pp, const std::vector<Segmen
 // thirtieth of a pass (14 us at 60M rows): the finish costs 38 where a last
 // pass that decodes costs 40, and each row has n * pairs / S^2 others in its
 // run, cheap while one thread sorts the run in registers (60M rows of about
-// six to a run: 0.54 ms) and dear beyond it (1M rows: the finish takes 15 us
+// six to a run: 0.56 ms) and dear beyond it (1M rows: the finish takes 15 us
 // at one or two rows to a run, 40 at 25, a pass 17).  Rows expected in runs of
 // more than 32 are never left to the finish.
 static int leading_digits(int bits, int64_t n, const unsigned long long* pairs, int S, int first) {
